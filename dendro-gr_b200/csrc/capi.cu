@@ -33,15 +33,6 @@ bool valid_side(int s) { return s == 13 || s == 19 || s == 31 || s == 55; }
 
 cudaStream_t S(bssn_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// the tile used before tuning: the split 7x7x7 brick (fastest on every
-// block size measured on B200)
-int default_tile() { return bssn::default_split_tile(); }
-
-int tile_for_side(const bssn::MeshState* m, int side) {
-    auto it = m->tuned.find(side);
-    return it == m->tuned.end() ? default_tile() : it->second;
-}
-
 }  // namespace
 
 extern "C" {
@@ -86,7 +77,7 @@ int bssn_bssnrhs_f64(double* const* rhs_dev, const double* const* u_dev, int64_t
         b.ptmin[d] = pmin[d];
         b.ptmax[d] = pmax[d];
     }
-    return bssn::launch_rhs_single(default_tile(), A, b, S(stream));
+    return bssn::launch_rhs_single(bssn::default_split_tile(b.sz), A, b, S(stream));
 }
 
 int bssn_mesh_create(const BssnBlockDesc* blocks, int nblocks, const int32_t G[3],
@@ -121,14 +112,33 @@ int bssn_rhs_blocks_f64(bssn_mesh mesh, double* const* rhs_dev, const double* co
         A.rhs.p[v] = rhs_dev[v];
     }
     A.prm = *params;
-    const int t = tile >= 0 ? tile : tile_for_side(mesh->st, 0);
-    const bssn::BrickTask* tasks;
-    int ntasks;
-    int r = bssn::mesh_tasks(mesh->st, t, &tasks, &ntasks);
-    if (!r) r = bssn::mesh_scratch(mesh->st, bssn::split_need(mesh->st, t, 0));
-    if (r) return r;
-    return bssn::launch_rhs_tasks(t, A, mesh->st->d_blocks, tasks, ntasks, S(stream),
-                                  mesh->st->d_scratch, mesh->st->scratch_zones);
+    A.axis = mesh->st->d_axis;
+    // every list and the scratch before the first launch: the split passes
+    // side by side (each with its default tile, or the one asked for), the
+    // single-kernel forms over all blocks at once
+    bssn::MeshState* m = mesh->st;
+    struct List {
+        int tile, side, ntasks;
+        const bssn::BrickTask* tasks;
+    };
+    std::vector<List> lists;
+    int64_t need = 0;
+    const std::vector<int> all{0};
+    const std::vector<int>& sides = tile < 0 || bssn::tile_mode(tile) == 1 ? m->sides : all;
+    for (int side : sides) {
+        List l;
+        l.side = side;
+        l.tile = tile >= 0 && bssn::tile_fits(tile, side) ? tile : bssn::default_split_tile(side);
+        const int r = bssn::mesh_tasks_side(m, l.tile, side, &l.tasks, &l.ntasks);
+        if (r) return r;
+        need = std::max(need, bssn::split_need(m, l.tile, side));
+        lists.push_back(l);
+    }
+    int r = bssn::mesh_scratch(m, need);
+    for (size_t k = 0; k < lists.size() && !r; k++)
+        r = bssn::launch_rhs_tasks(lists[k].tile, lists[k].side, A, m->d_blocks, lists[k].tasks, lists[k].ntasks, S(stream),
+                                   m->d_scratch, m->scratch_zones);
+    return r;
 }
 
 int bssn_unzip_f64(bssn_mesh mesh, double* const* unzip_dev, const double* const* zip_dev,

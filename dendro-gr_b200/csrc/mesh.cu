@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <set>
 #include <vector>
 
 #include "bssn_common.cuh"
@@ -121,6 +122,9 @@ int mesh_create(const BssnBlockDesc* blocks, int nblocks, const int32_t G[3],
         const int64_t s = blocks[b].sz;
         m->unzip_size = std::max<int64_t>(m->unzip_size, blocks[b].offset + s * s * s);
     }
+    std::set<int> sides;
+    for (auto& b : m->blocks) sides.insert(b.sz);
+    m->sides.assign(sides.begin(), sides.end());
     std::vector<Chunk> pad, inner, small;
     make_chunks(m->blocks, false, pad);
     make_chunks(m->blocks, true, inner);
@@ -129,6 +133,10 @@ int mesh_create(const BssnBlockDesc* blocks, int nblocks, const int32_t G[3],
     m->n_int_chunks = (int)inner.size();
     m->n_pad_chunks_small = (int)small.size();
     int st = upload(m->blocks, &m->d_blocks);
+    std::vector<AxisCoef> axis;
+    for (auto& b : m->blocks)
+        for (int d = 0; d < 3; d++) axis.push_back(axis_coef((b.ptmax[d] - b.ptmin[d]) / (b.sz - 1)));
+    if (!st) st = upload(axis, &m->d_axis);
     if (!st) st = upload(pad, &m->d_pad_chunks);
     if (!st) st = upload(inner, &m->d_int_chunks);
     if (!st) st = upload(small, &m->d_pad_chunks_small);
@@ -143,6 +151,7 @@ int mesh_create(const BssnBlockDesc* blocks, int nblocks, const int32_t G[3],
 void mesh_destroy(MeshState* m) {
     if (!m) return;
     cudaFree(m->d_blocks);
+    cudaFree(m->d_axis);
     cudaFree(m->d_pad_chunks);
     cudaFree(m->d_pad_chunks_small);
     cudaFree(m->d_int_chunks);
@@ -182,7 +191,7 @@ int64_t split_need(MeshState* m, int tile, int side) {
     const BrickTask* tk;
     int nt = 0;
     if (mesh_tasks_side(m, tile, side, &tk, &nt)) return 0;
-    const int64_t need = (int64_t)nt * tile_zones(tile);
+    const int64_t need = (int64_t)nt * tile_zones(tile, side);
     return need < kSplitScratchZonesMax ? need : kSplitScratchZonesMax;
 }
 
@@ -206,12 +215,7 @@ int mesh_tasks_side(MeshState* m, int tile, int side, const BrickTask** tasks, i
         std::vector<BrickTask> all, h;
         build_tasks(m->blocks.data(), (int)m->blocks.size(), tile, all);
         for (auto& t : all)
-            if (side <= 0 || m->blocks[t.blk].sz == side) h.push_back(t);
-        if (side < 0) {  // all blocks, Z-order of their origins (bricks of a block stay together)
-            std::stable_sort(h.begin(), h.end(), [&](const BrickTask& a, const BrickTask& b) {
-                return morton_key(m->blocks[a.blk]) < morton_key(m->blocks[b.blk]);
-            });
-        }
+            if (side == 0 || m->blocks[t.blk].sz == side) h.push_back(t);
         BrickTask* d = nullptr;
         int st = upload(h, &d);
         if (st) return st;
@@ -244,10 +248,6 @@ int mesh_partition(const BssnBlockDesc* blocks, int nblocks, int nparts, int32_t
         acc += z;
     }
     return 0;
-}
-
-int mesh_tasks(MeshState* m, int tile, const BrickTask** tasks, int* ntasks) {
-    return mesh_tasks_side(m, tile, 0, tasks, ntasks);
 }
 
 int launch_unzip(const MeshState* m, double* const* unz, const double* const* zip,

@@ -19,6 +19,7 @@ namespace bssn {
 // tile is a stack of short rows in a padded block of that size anyway, so
 // reading the node grid costs no more and their ghost fill is skipped.
 constexpr int kDirectMinSide = 55;
+constexpr int kAllSides = -1;
 
 // A run of consecutive points of one block handled by one CTA.
 struct Chunk {
@@ -29,9 +30,11 @@ struct Chunk {
 
 struct MeshState {
     std::vector<BssnBlockDesc> blocks;
+    std::vector<int> sides;  // padded sides present, ascending
     int32_t G[3];
     int64_t unzip_size;
     BssnBlockDesc* d_blocks = nullptr;
+    AxisCoef* d_axis = nullptr;  // stencil factors of every block and axis
     Chunk* d_pad_chunks = nullptr;
     Chunk* d_int_chunks = nullptr;
     int n_pad_chunks = 0;
@@ -60,7 +63,8 @@ struct MeshState {
     int64_t* d_fchunk_first = nullptr;
     double* d_fpart = nullptr;
     int n_fchunks = 0;
-    // autotuned tile per padded side (0 = not tuned)
+    // autotuned or pinned tile per padded side, or (direct plans) one for
+    // every side under the key kAllSides
     std::map<int, int> tuned;
     // scratch of the split right-hand side (kSplitSlots doubles per zone)
     double* d_scratch = nullptr;
@@ -73,11 +77,8 @@ struct MeshState {
 int mesh_create(const BssnBlockDesc* blocks, int nblocks, const int32_t G[3],
                 MeshState** out);
 void mesh_destroy(MeshState* m);
-int mesh_tasks(MeshState* m, int tile, const BrickTask** tasks, int* ntasks);
-// Brick tasks of one tile for the blocks of padded side `side` (in block
-// order), for all blocks (side 0, block order) or for all blocks in the
-// Z-order of their origins (side kAllZOrder).
-constexpr int kAllZOrder = -1;
+// Brick tasks of one tile for the blocks of padded side `side`, or for all
+// blocks (side 0), in block order.
 int mesh_tasks_side(MeshState* m, int tile, int side, const BrickTask** tasks, int* ntasks);
 // Make the split-path scratch hold at least min(zones, kSplitScratchZonesMax)
 // zones (allocates; call outside stream capture).

@@ -9,7 +9,6 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
-#include <set>
 #include <vector>
 
 #include "bssn_b200.h"
@@ -35,6 +34,13 @@ void set_ptrs(double* base, int64_t n, double* out[NVARS]) {
 }
 
 }  // namespace
+
+// Whether a plan can run a tile on its blocks of padded side `side`: direct
+// plans need a kernel that reads and writes the zipped grid, and a split
+// tile's brick must not be wider than the block.
+static bool plan_runs_tile(const Plan* p, int tile, int side) {
+    return tile_fits(tile, side) && (!p->direct || tile_zipped(tile_mode(tile)));
+}
 
 int plan_create(MeshState* m, const BssnParams& prm, int flags, Plan** out) {
     Plan* p = new Plan();
@@ -70,18 +76,14 @@ int plan_create(MeshState* m, const BssnParams& prm, int flags, Plan** out) {
         plan_destroy(p);
         return st;
     }
-    std::set<int> sides;
-    for (auto& b : m->blocks) sides.insert(b.sz);
-    p->sides.assign(sides.begin(), sides.end());
+    p->sides = m->sides;
     // task lists, the split-path scratch and kernel attributes must exist
     // before any graph capture
     int64_t need = 0;
-    // direct plans: one Z-ordered list over all blocks per split tile;
-    // padded plans: one list per block-size bucket and tile
-    std::vector<int> keys = p->direct ? std::vector<int>{kAllZOrder} : p->sides;
-    for (int key : keys) {
+    // one list per block-size bucket and tile
+    for (int key : p->sides) {
         for (int t = 0; t < tile_count(); t++) {
-            if (p->direct && !tile_zipped(tile_mode(t))) continue;
+            if (!plan_runs_tile(p, t, key)) continue;
             const BrickTask* tk;
             int nt;
             st = mesh_tasks_side(m, t, key, &tk, &nt);
@@ -136,21 +138,20 @@ void plan_destroy(Plan* p) {
     delete p;
 }
 
-// The tile a plan runs for blocks of side `side`: direct plans run one split
-// tile over all blocks (tuned under the key kAllZOrder), padded plans the
-// tile tuned for the side.
+// The tile a plan runs for blocks of side `side`: the one tuned or pinned for
+// it (direct plans: for all sides, under the key kAllSides) where it can run
+// it, else the side's default.
 int plan_tile(const Plan* p, int side) {
-    auto it = p->mesh->tuned.find(p->direct ? kAllZOrder : side);
+    auto it = p->mesh->tuned.find(p->direct ? kAllSides : side);
     const int t = it == p->mesh->tuned.end() ? -1 : it->second;
-    if (p->direct) return (t >= 0 && tile_zipped(tile_mode(t))) ? t : default_split_tile();
-    return t >= 0 ? t : default_split_tile();
+    return t >= 0 && plan_runs_tile(p, t, side) ? t : default_split_tile(side);
 }
 
 int plan_set_tile(Plan* p, int side, int tile) {
     if (tile < 0 || tile >= tile_count()) return BSSN_EINVAL;
     if (p->direct) {
         if (!tile_zipped(tile_mode(tile))) return BSSN_EINVAL;
-        p->mesh->tuned[kAllZOrder] = tile;
+        p->mesh->tuned[kAllSides] = tile;
     } else if (side == 0) {
         for (int sd : p->sides) p->mesh->tuned[sd] = tile;
     } else {
@@ -177,6 +178,7 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
     MeshState* m = p->mesh;
     RhsArgs A;
     A.prm = p->prm;
+    A.axis = m->d_axis;
     if (p->direct) {
         double* Rz[NVARS];
         set_ptrs(p->Rz, p->n_nodes, Rz);
@@ -184,13 +186,17 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
             A.u.p[v] = src[v];
             A.rhs.p[v] = Rz[v];
         }
-        const int t = plan_tile(p, kAllZOrder);
-        const BrickTask* tk;
-        int nt;
-        int st = mesh_tasks_side(m, t, kAllZOrder, &tk, &nt);
-        if (!st)
-            st = launch_rhs_tasks(t, A, m->d_blocks, tk, nt, s, m->d_scratch, m->scratch_zones, tm,
-                                  m->G);
+        int st = 0;
+        for (int side : p->sides) {
+            const int t = plan_tile(p, side);
+            const BrickTask* tk;
+            int nt;
+            st = mesh_tasks_side(m, t, side, &tk, &nt);
+            if (!st)
+                st = launch_rhs_tasks(t, side, A, m->d_blocks, tk, nt, s, m->d_scratch, m->scratch_zones, tm,
+                                      m->G);
+            if (st) break;
+        }
         return st;
     }
     double* Pp[NVARS];
@@ -222,7 +228,7 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
                 const int per = bricks_per_block(t, b.sz);
                 if (!st && (j + 1) * per > nt) st = BSSN_ESTATE;
                 if (!st)
-                    st = launch_rhs_tasks(t, A, m->d_blocks, tk + (size_t)j * per, per, s, m->d_scratch,
+                    st = launch_rhs_tasks(t, b.sz, A, m->d_blocks, tk + (size_t)j * per, per, s, m->d_scratch,
                                           m->scratch_zones, tm);
             } else {
                 st = launch_rhs_single(t, A, b, s);
@@ -243,7 +249,7 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
         int st = mesh_tasks_side(m, t, side, &tk, &nt);
         const bool direct = zrhs && src && side >= kDirectMinSide;
         if (!st)
-            st = launch_rhs_tasks(t, direct ? Ad : A, m->d_blocks, tk, nt, s, m->d_scratch,
+            st = launch_rhs_tasks(t, side, direct ? Ad : A, m->d_blocks, tk, nt, s, m->d_scratch,
                                   m->scratch_zones, tm, zrhs ? m->G : nullptr, direct);
         if (st) return st;
     }
@@ -424,6 +430,7 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
     MeshState* m = p->mesh;
     RhsArgs A;
     A.prm = p->prm;
+    A.axis = m->d_axis;
     int st = 0;
     if (p->direct) {  // split tiles on the zipped state u
         double* Rz[NVARS];
@@ -449,34 +456,48 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const int nt = tile_count();
+    // milliseconds of one pass of a tile over the blocks of one side
+    auto time_tile = [&](int t, int side, float& ms) {
+        const BrickTask* tk;
+        int ntask;
+        int r = mesh_tasks_side(m, t, side, &tk, &ntask);
+        ms = 1e30f;
+        for (int k = 0; k <= reps && !r; k++) {
+            cudaEventRecord(e0, s);
+            r = launch_rhs_tasks(t, side, A, m->d_blocks, tk, ntask, s, m->d_scratch, m->scratch_zones, nullptr, zg);
+            cudaEventRecord(e1, s);
+            if (r) break;
+            cudaEventSynchronize(e1);
+            float x = 0;
+            cudaEventElapsedTime(&x, e0, e1);
+            if (k > 0) ms = std::min(ms, x);
+        }
+        return r;
+    };
     if (p->direct) {
-        // every split tile over the whole Z-ordered list; each bucket row of
-        // `times` gets the same figures
+        // one tile for every side: the fastest over all of them (where a side
+        // cannot run it, its default); each bucket row of `times` gets the
+        // same figures
         float best = 1e30f;
-        int best_t = default_split_tile();
+        int best_t = -1;
         std::vector<float> tt(nt, 1e30f);
         for (int t = 0; t < nt && !st; t++) {
             if (!tile_zipped(tile_mode(t))) continue;
-            const BrickTask* tk;
-            int ntask;
-            st = mesh_tasks_side(m, t, kAllZOrder, &tk, &ntask);
-            for (int r = 0; r <= reps && !st; r++) {
-                cudaEventRecord(e0, s);
-                st = launch_rhs_tasks(t, A, m->d_blocks, tk, ntask, s, m->d_scratch,
-                                      m->scratch_zones, nullptr, zg);
-                cudaEventRecord(e1, s);
-                if (st) break;
-                cudaEventSynchronize(e1);
+            float sum = 0;
+            for (int side : p->sides) {
                 float ms = 0;
-                cudaEventElapsedTime(&ms, e0, e1);
-                if (r > 0) tt[t] = std::min(tt[t], ms);
+                st = time_tile(plan_runs_tile(p, t, side) ? t : default_split_tile(side), side, ms);
+                if (st) break;
+                sum += ms;
             }
-            if (!st && tt[t] < best) {
-                best = tt[t];
+            if (st) break;
+            tt[t] = sum;
+            if (sum < best) {
+                best = sum;
                 best_t = t;
             }
         }
-        if (!st) m->tuned[kAllZOrder] = best_t;
+        if (!st && best_t >= 0) m->tuned[kAllSides] = best_t;
         if (times_out)
             for (size_t i = 0; i < p->sides.size(); i++)
                 for (int t = 0; t < nt; t++) times_out[i * nt + t] = tt[t];
@@ -491,20 +512,7 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
         int best_t = 0;
         for (int t = 0; t < nt; t++) {
             float tbest = 1e30f;
-            const BrickTask* tk;
-            int ntask;
-            st = mesh_tasks_side(m, t, side, &tk, &ntask);
-            if (st) break;
-            for (int r = 0; r <= reps; r++) {
-                cudaEventRecord(e0, s);
-                st = launch_rhs_tasks(t, A, m->d_blocks, tk, ntask, s, m->d_scratch, m->scratch_zones);
-                cudaEventRecord(e1, s);
-                if (st) break;
-                cudaEventSynchronize(e1);
-                float ms = 0;
-                cudaEventElapsedTime(&ms, e0, e1);
-                if (r > 0) tbest = std::min(tbest, ms);
-            }
+            if (plan_runs_tile(p, t, side)) st = time_tile(t, side, tbest);
             if (st) break;
             if (times_out) times_out[idx * nt + t] = tbest;
             if (tbest < best) {
@@ -584,19 +592,13 @@ int plan_launches_per_step(Plan* p) {
     int rhs = 0;
     if (p->flags & BSSN_PLAN_PER_BLOCK) {
         for (auto& b : m->blocks) rhs += tile_mode(plan_tile(p, b.sz)) == 1 ? 2 : 1;
-    } else if (p->direct) {
-        const int t = plan_tile(p, kAllZOrder);
-        const BrickTask* tk;
-        int nt = 0;
-        if (mesh_tasks_side(m, t, kAllZOrder, &tk, &nt)) return -1;
-        rhs = rhs_launch_count(t, nt, m->scratch_zones);
     } else {
         for (int side : p->sides) {
             const int t = plan_tile(p, side);
             const BrickTask* tk;
             int nt = 0;
             if (mesh_tasks_side(m, t, side, &tk, &nt)) return -1;
-            rhs += rhs_launch_count(t, nt, m->scratch_zones);
+            rhs += rhs_launch_count(t, nt, m->scratch_zones, side);
         }
     }
     if (m->lv) {  // interpolation passes, ghost fill, stage, one launch per non-empty sync segment

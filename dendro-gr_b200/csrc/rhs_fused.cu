@@ -115,10 +115,11 @@ TileEntry make_fused(int id) {
     using Bk = Brick<BX, BY, BZ>;
     return TileEntry{BX, BY, BZ, Bk::THREADS, Bk::SMEM_BYTES, rhs_kernel<BX, BY, BZ, 1>, 0, -1, id};
 }
-template <int BX, int BY, int BZ>
+// split: columns of the shape, every brick as high as its block
 TileEntry make_split_tile(int shape, int fused) {
-    using Bk = Brick<BX, BY, BZ>;
-    return TileEntry{BX, BY, BZ, Bk::THREADS, Bk::SMEM_BYTES, nullptr, 1, shape, fused};
+    int b[2];
+    split_columns(shape, b);
+    return TileEntry{b[0], b[1], 49, split_threads(shape), split_smem(shape), nullptr, 1, shape, fused};
 }
 template <int BX, int BY, int BZ>
 TileEntry make_onchip_tile(int shape) {
@@ -126,29 +127,34 @@ TileEntry make_onchip_tile(int shape) {
     return TileEntry{BX, BY, BZ, Bk::THREADS, 0, nullptr, 2, shape, -1};
 }
 
-// tiles 0..2: fused; 3..5: the same shapes split; 6..9: split-only shapes
-// (13x5x5 and 9x9x5 fit the 25-zone interiors of 31^3 blocks with few idle
-// threads); 10..13: on chip (128-zone bricks, every extent >= 3 for every
-// block side, as the one-sided closures need; 10, 11 at two CTAs per SM,
-// 12, 13 the same shapes at three)
-// (rhs_split.cu's shape order).  `fused` is the tile a single-block launch
-// of the shape runs (the nearest fused shape for split-only ones).
+// tiles 0..2: fused; 3..9: split (13x5 and 9x9 columns fit the 25-zone
+// interiors of 31^3 blocks with few idle threads; 6 and 7 repeat the columns
+// of 4 and 3, from which only their heights once told them apart); 10..13: on
+// chip (128-zone bricks, every extent >= 3 for every block side, as the
+// one-sided closures need; 10, 11 at two CTAs per SM, 12, 13 the same shapes
+// at three); 14..16: split, whole layers or full-width strips of one block
+// side each (the defaults of sides 19, 31, 55).  `fused` is the tile a
+// single-block launch of the shape runs (the nearest fused shape for
+// split-only ones).
 const TileEntry* tile_table(int* count) {
     static const TileEntry table[] = {
         make_fused<8, 8, 4>(0),
         make_fused<7, 7, 4>(1),
         make_fused<8, 4, 4>(2),
-        make_split_tile<8, 8, 4>(0, 0),
-        make_split_tile<7, 7, 4>(1, 1),
-        make_split_tile<8, 4, 4>(2, 2),
-        make_split_tile<7, 7, 7>(3, 1),
-        make_split_tile<8, 8, 8>(4, 0),
-        make_split_tile<13, 5, 5>(5, 1),
-        make_split_tile<9, 9, 5>(6, 1),
+        make_split_tile(0, 0),
+        make_split_tile(1, 1),
+        make_split_tile(2, 2),
+        make_split_tile(1, 1),
+        make_split_tile(0, 0),
+        make_split_tile(3, 1),
+        make_split_tile(4, 1),
         make_onchip_tile<5, 5, 5>(0),
         make_onchip_tile<7, 4, 4>(1),
         make_onchip_tile<5, 5, 5>(2),
         make_onchip_tile<7, 4, 4>(3),
+        make_split_tile(5, 1),
+        make_split_tile(6, 1),
+        make_split_tile(7, 1),
     };
     *count = (int)(sizeof(table) / sizeof(table[0]));
     return table;
@@ -177,22 +183,23 @@ int tile_mode(int tile) {
     return (tile < 0 || tile >= c) ? -1 : tab[tile].mode;
 }
 
-int default_split_tile() {
+// The split tile a block side runs before tuning: whole layers of the block,
+// or for 55^3 the widest strip whose columns a CTA's threads hold.  A brick
+// pays its halo columns and rows once, so the largest one is the fastest.
+int default_split_tile(int side) { return side == 19 ? 14 : side == 31 ? 15 : side == 55 ? 16 : 6; }
+
+int tile_zones(int tile, int side) {
     int c;
     const TileEntry* tab = tile_table(&c);
-    int first = -1;
-    for (int t = 0; t < c; t++) {
-        if (tab[t].mode != 1) continue;
-        if (first < 0) first = t;
-        if (tab[t].bx == 7 && tab[t].by == 7 && tab[t].bz == 7) return t;
-    }
-    return first;
+    return (tile < 0 || tile >= c) ? 0 : tab[tile].bx * tab[tile].by * (side - 2 * PW);
 }
 
-int tile_zones(int tile) {
+bool tile_fits(int tile, int side) {
     int c;
     const TileEntry* tab = tile_table(&c);
-    return (tile < 0 || tile >= c) ? 0 : tab[tile].bx * tab[tile].by * tab[tile].bz;
+    if (tile < 0 || tile >= c) return false;
+    // bricks of the small shapes clip to any block
+    return tab[tile].mode != 1 || tab[tile].bx <= 13 || tab[tile].bx <= side - 2 * PW;
 }
 
 // Host replay of the brick kernel's shared-memory indexing: for a tile
@@ -279,7 +286,7 @@ long tile_selfcheck(int tile) {
     int c;
     const TileEntry* tab = tile_table(&c);
     if (tile < 0 || tile >= c) return -1;
-    // split tiles stage and read their tiles as fused tiles of the shape do
+    if (tab[tile].mode == 1) return split_selfcheck(tab[tile].shape);
     const int b[3] = {tab[tile].bx, tab[tile].by, tab[tile].bz};
     auto is = [&](int x, int y, int z) { return b[0] == x && b[1] == y && b[2] == z; };
     if (is(8, 8, 4)) return check_tile_shape<8, 8, 4>();
@@ -287,10 +294,6 @@ long tile_selfcheck(int tile) {
     if (is(7, 4, 4)) return check_tile_shape<7, 4, 4>();
     if (is(7, 7, 4)) return check_tile_shape<7, 7, 4>();
     if (is(8, 4, 4)) return check_tile_shape<8, 4, 4>();
-    if (is(7, 7, 7)) return check_tile_shape<7, 7, 7>();
-    if (is(8, 8, 8)) return check_tile_shape<8, 8, 8>();
-    if (is(13, 5, 5)) return check_tile_shape<13, 5, 5>();
-    if (is(9, 9, 5)) return check_tile_shape<9, 9, 5>();
     return -1;
 }
 
@@ -333,7 +336,7 @@ void build_tasks(const BssnBlockDesc* blocks, int nblocks, int tile,
     }
 }
 
-int launch_rhs_tasks(int tile, const RhsArgs& A, const BssnBlockDesc* blocks_dev,
+int launch_rhs_tasks(int tile, int side, const RhsArgs& A, const BssnBlockDesc* blocks_dev,
                      const BrickTask* tasks_dev, int ntasks, cudaStream_t s,
                      double* scratch, int64_t scratch_zones, KernelTimer* tm,
                      const int32_t* zip_grid, bool zip_in) {
@@ -344,7 +347,7 @@ int launch_rhs_tasks(int tile, const RhsArgs& A, const BssnBlockDesc* blocks_dev
     const TileEntry& t = tab[tile];
     if (t.mode == 1)
         return launch_rhs_split(t.shape, A, blocks_dev, tasks_dev, ntasks, scratch, scratch_zones,
-                                s, tm, zip_grid, zip_in);
+                                s, tm, zip_grid, zip_in, side);
     if (t.mode == 2)
         return launch_rhs_onchip(t.shape, A, blocks_dev, tasks_dev, ntasks, s, tm, zip_grid, zip_in);
     if (zip_grid) return BSSN_EINVAL;  // the fused kernel writes padded right-hand sides only
@@ -366,10 +369,10 @@ int bricks_per_block(int tile, int side) {
     return ((n + t.bx - 1) / t.bx) * ((n + t.by - 1) / t.by) * ((n + t.bz - 1) / t.bz);
 }
 
-int rhs_launch_count(int tile, int ntasks, int64_t scratch_zones) {
+int rhs_launch_count(int tile, int ntasks, int64_t scratch_zones, int side) {
     if (ntasks <= 0) return 0;
     if (tile_mode(tile) != 1) return 1;
-    const int64_t chunk = scratch_zones / tile_zones(tile);
+    const int64_t chunk = scratch_zones / tile_zones(tile, side);
     return chunk > 0 ? (int)(2 * ((ntasks + chunk - 1) / chunk)) : 0;
 }
 

@@ -14,6 +14,7 @@ struct RhsArgs {
     ConstVars u;
     MutVars rhs;
     BssnParams prm;
+    const AxisCoef* axis = nullptr;  // stencil factors, three per block of the list's mesh (split tiles)
 };
 
 // One brick: block index, interior origin and extent per axis.
@@ -36,8 +37,12 @@ int tile_count();
 int tile_mode(int tile);   // 0 fused, 1 split, 2 on chip, -1 unknown
 // whether a tile's kernels can write zipped right-hand sides (split, on chip)
 inline bool tile_zipped(int mode) { return mode == 1 || mode == 2; }
-int default_split_tile();  // the split tile used before autotuning
-int tile_zones(int tile);  // zones per brick (BX*BY*BZ)
+int default_split_tile(int side);  // the split tile of a block side before autotuning
+// zones per brick of a split tile on blocks of padded side `side`
+int tile_zones(int tile, int side);
+// whether a tile runs on blocks of padded side `side`: not when its brick is
+// wider than their interior
+bool tile_fits(int tile, int side);
 long tile_selfcheck(int tile);
 int prepare_all_tiles();
 int tile_info(int tile, int info[4]);
@@ -89,7 +94,9 @@ struct KernelTimer {
 // per node by the block owning it (zones that do not own their node are
 // skipped), and A.u the zipped stage state (zip_in, direct form) or the
 // padded one.
-int launch_rhs_tasks(int tile, const RhsArgs& A, const BssnBlockDesc* blocks_dev,
+// side: the padded side of every block of the list (0: several sides, not
+// for split tiles).
+int launch_rhs_tasks(int tile, int side, const RhsArgs& A, const BssnBlockDesc* blocks_dev,
                      const BrickTask* tasks_dev, int ntasks, cudaStream_t s,
                      double* scratch, int64_t scratch_zones, KernelTimer* tm = nullptr,
                      const int32_t* zip_grid = nullptr, bool zip_in = true);
@@ -97,7 +104,7 @@ int launch_rhs_tasks(int tile, const RhsArgs& A, const BssnBlockDesc* blocks_dev
 // a block's bricks together, blocks in mesh order)
 int bricks_per_block(int tile, int side);
 // kernel launches launch_rhs_tasks makes for a task list of ntasks bricks
-int rhs_launch_count(int tile, int ntasks, int64_t scratch_zones);
+int rhs_launch_count(int tile, int ntasks, int64_t scratch_zones, int side);
 // one block; a split tile runs its shape fused
 int launch_rhs_single(int tile, const RhsArgs& A, const BssnBlockDesc& blk,
                       cudaStream_t s);
@@ -113,11 +120,14 @@ int launch_rhs_onchip_single(int shape, const RhsArgs& A, const BssnBlockDesc& b
 
 // split path (rhs_split.cu); shape = index among the split shapes
 int split_shape_count();
-int split_zone_count(int shape);
+int split_columns(int shape, int b[2]);  // columns of a brick
+int split_threads(int shape);    // of the derivative pass
+size_t split_smem(int shape);
+long split_selfcheck(int shape);  // host replay of its shared-memory indexing
 int prepare_split(int shape);
 int launch_rhs_split(int shape, const RhsArgs& A, const BssnBlockDesc* blocks_dev,
                      const BrickTask* tasks_dev, int ntasks, double* scratch,
-                     int64_t scratch_zones, cudaStream_t s, KernelTimer* tm = nullptr,
-                     const int32_t* zip_grid = nullptr, bool zip_in = true);
+                     int64_t scratch_zones, cudaStream_t s, KernelTimer* tm,
+                     const int32_t* zip_grid, bool zip_in, int side);
 
 }  // namespace bssn

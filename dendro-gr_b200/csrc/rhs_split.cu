@@ -1,28 +1,29 @@
 // Split BSSN right-hand side: a derivative pass, then a pointwise equation
-// pass, over the same brick task lists as the fused kernel.
+// pass, over brick task lists.
 //
 // The fused kernel keeps every derivative of a zone in registers; its code is
 // one straight run of all 24 variables (about 1 MB of instructions) at 255
 // registers and one CTA per SM, so it stalls on instruction fetch and on
 // FP64 latency.  Here:
-//   * deriv_kernel loops over the 24 variables at run time (one copy of the
-//     staging, mixed-pass and stencil code), at a few dozen registers and
-//     several CTAs per SM, and writes each zone's gradient, second
-//     derivatives and summed KO term to a scratch array;
+//   * column_kernel (rhs_columns.cuh) marches columns of each variable along
+//     z and writes every zone's gradient, second derivatives and summed KO
+//     term to a scratch array;
 //   * eq_kernel evaluates the equations per zone (rhs_equations.cuh, the same
 //     code as the fused kernel) reading those derivatives back.
-// The scratch holds slot pairs, [slot / 2][task * NZ + thread][slot % 2]
-// (every variable has an even number of slots), so both passes move 16-byte
-// pairs in whole rows of consecutive zones.  A task list longer than the scratch is
-// processed in chunks, each a derivative launch followed by an equation
-// launch on the same stream.
+// The scratch holds slot pairs, [pair][task * NZ + zone][2], so both passes
+// move 16-byte pairs in whole rows of consecutive zones.  A task list longer
+// than the scratch is processed in chunks, each a derivative launch followed
+// by an equation launch on the same stream.
 //
-// Derivatives are bit-identical to the fused kernel's (same stencils, same
-// tiles); the equations are the same code, so both paths give the same RHS.
+// Derivatives are bit-identical to the fused kernel's (same stencils); the
+// equations are the same code, so both paths give the same RHS.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "bssn_common.cuh"
 #include "rhs_brick.cuh"
+#include "rhs_columns.cuh"
 #include "rhs_equations.cuh"
 #include "rhs_fused.cuh"
 
@@ -30,150 +31,17 @@ namespace bssn {
 
 namespace {
 
-// Scratch slots per zone: gradient (3) + second derivatives (6) + KO for the
-// 11 variables with second derivatives, gradient + KO for the other 13.
-constexpr int kSlotsSecond = 10;
-constexpr int kSlotsFirst = 4;
-__host__ __device__ constexpr int slot_len(int step) {
-    return stage_second(step) ? kSlotsSecond : kSlotsFirst;
-}
-__host__ __device__ constexpr int slot_base(int step) {
-    int b = 0;
-    for (int k = 0; k < step; k++) b += slot_len(k);
-    return b;
-}
-static_assert(slot_base(NVARS) == kSplitSlots, "scratch slot count");
-
-// resident derivative CTAs per SM the register allocation must allow: 3 for
-// up to 384 threads (56 registers at 352), 2 for up to 512, else 1
-__host__ __device__ constexpr int deriv_min_ctas(int threads) {
-    return threads <= 384 ? 3 : threads <= 512 ? 2 : 1;
-}
 // equation pass: variables whose derivatives are in flight ahead of use, and
-// the per-thread ring of scratch slots (shared memory) they land in; one
+// the per-thread ring of scratch pairs (shared memory) they land in; one
 // variable more than the prefetch distance, so a copy never targets a row
 // read by the variable just consumed
 constexpr int kPrefetchSteps = 6;
-constexpr int kRingSlots = (kPrefetchSteps + 1) * kSlotsSecond;
-constexpr int kRingPairs = kRingSlots / 2;
+constexpr int kRingPairs = (kPrefetchSteps + 1) * kPairsSecond;
 constexpr int kEqThreads = 128;
-// derivative pass: shared-memory tiles (variables staged kDerivBuffers - 1 ahead)
-constexpr int kDerivBuffers = 2;
-template <class Bk>
-constexpr size_t deriv_smem_bytes() {
-    return sizeof(double) * (kDerivBuffers * Bk::TILE + Bk::MXJ + 2 * Bk::MXK);
-}
 
 template <int N>
 __device__ __forceinline__ void cp_async_wait_pending() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-// Whether the zone at brick position t owns its node of the zipped grid: a
-// node on a block's upper face belongs to the next block unless the face
-// lies on the grid's upper boundary (the zip's owner rule).
-__device__ __forceinline__ bool owns_node(const BssnBlockDesc& blk, const int o[3], const int t[3],
-                                          const ZipGrid& g) {
-    const int n = blk.sz - 2 * PW;
-    const int gd[3] = {g.gx, g.gy, g.gz};
-    bool own = true;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const int i = o[d] + t[d];  // interior index
-        own = own && (i < n - 1 || blk.g0[d] + i == gd[d] - 1);
-    }
-    return own;
-}
-
-// ZIP: stage from the zipped node grid (g) instead of the padded blocks.
-template <int BX, int BY, int BZ, bool ZIP>
-__global__ void __launch_bounds__(Brick<BX, BY, BZ>::THREADS,
-                                   deriv_min_ctas(Brick<BX, BY, BZ>::THREADS))
-deriv_kernel(ConstVars u, const BssnBlockDesc* __restrict__ blocks,
-             const BrickTask* __restrict__ tasks, double* __restrict__ S, int64_t zs,
-             ZipGrid g) {
-    using Bk = Brick<BX, BY, BZ>;
-    extern __shared__ __align__(16) double smem[];
-    __shared__ const double* src[NVARS];
-    __shared__ AxisCoef cfs[3];
-    double* tiles = smem;                         // kDerivBuffers tiles
-    double* mx = smem + kDerivBuffers * Bk::TILE;  // mxj | mxk | myk
-    const BrickTask tk = tasks[blockIdx.x];
-    const BssnBlockDesc blk = blocks[tk.blk];
-    const int o[3] = {tk.o[0], tk.o[1], tk.o[2]};
-    const int e[3] = {tk.e[0], tk.e[1], tk.e[2]};
-    const int tid = threadIdx.x;
-    const int s = blk.sz;
-    if (tid < NVARS) src[tid] = u.p[stage_order(tid)] + (ZIP ? 0 : blk.offset);
-    fill_axis_coefs(cfs, blk, tid);
-    const BrickThread<Bk> th(tid, e);
-    const BrickZone<Bk> bz(blk, o, th, cfs);
-    const StagePlan<Bk, ZIP> sp(o, e, s, tid, g, blk.g0);
-    // zones whose derivatives the equation pass reads: every zone of the
-    // brick, or (node grid given: direct form or stage mode) only the zones
-    // that own their node
-    const bool keep = th.active && (g.gx == 0 || owns_node(blk, o, th.t, g));
-    // next scratch slot pair of this zone (kept zones only advance it)
-    double2* w = reinterpret_cast<double2*>(S) + (int64_t)blockIdx.x * Bk::NZ + tid;
-    __syncthreads();
-
-    // variables in flight kDerivBuffers - 1 ahead; one commit group per
-    // variable (empty past the last one, so the pending count stays fixed)
-#pragma unroll
-    for (int k = 0; k < kDerivBuffers - 1; k++) sp.stage(src[k], tiles + k * Bk::TILE, tid);
-#pragma unroll 1
-    for (int step = 0; step < NVARS; step++) {
-        cp_async_wait_pending<kDerivBuffers - 2>();
-        __syncthreads();  // the tile of `step` is complete; the buffer below was last read at step - 1
-        const double* cur = tiles + (step % kDerivBuffers) * Bk::TILE;
-        const int nxt = step + kDerivBuffers - 1;
-        if (nxt < NVARS)
-            sp.stage(src[nxt], tiles + (nxt % kDerivBuffers) * Bk::TILE, tid);
-        else
-            cp_async_commit();
-        if (stage_second(step)) {
-            Dir3 r[3];
-            zone_dirs<true, Bk>(bz.zc, cur, r);
-            // the brick part of the mixed scratch from the zones' own gradient
-            if (th.active) {
-                mx[bz.mxj_off] = r[0].d1;  // the offsets include the halo
-                mx[Bk::MXJ + bz.mxk_off] = r[0].d1;
-                mx[Bk::MXJ + Bk::MXK + bz.mxk_off] = r[1].d1;
-            }
-            mixed_halo_pass<Bk>(cur, mx, o, e, s, blk.bflag, bz.zc.cf, tid);
-            __syncthreads();
-            const double* mxj = mx + bz.mxj_off;
-            const double* mxk = mx + Bk::MXJ + bz.mxk_off;
-            const double* myk = mx + Bk::MXJ + Bk::MXK + bz.mxk_off;
-            const ZoneCtx& z = bz.zc;
-            double xy = d1_fast_in(mxj, Bk::BX, z.cf[1]);
-            double xz = d1_fast_in(mxk, Bk::BX * Bk::BY, z.cf[2]);
-            double yz = d1_fast_in(myk, Bk::BX * Bk::BY, z.cf[2]);
-            if (z.bflag) {
-                if (near_face(z.a[1], s, z.bflag & 4u, z.bflag & 8u))
-                    xy = closure_d1(mxj, bz.mj, z.a[1], s, z.bflag & 4u, z.cf[1]);
-                if (near_face(z.a[2], s, z.bflag & 16u, z.bflag & 32u)) {
-                    xz = closure_d1(mxk, bz.mk, z.a[2], s, z.bflag & 16u, z.cf[2]);
-                    yz = closure_d1(myk, bz.mk, z.a[2], s, z.bflag & 16u, z.cf[2]);
-                }
-            }
-            if (keep) {
-                const double v[kSlotsSecond] = {r[0].d1, r[1].d1, r[2].d1, r[0].d2, xy, xz,
-                                                r[1].d2, yz, r[2].d2, r[0].ko + r[1].ko + r[2].ko};
-#pragma unroll
-                for (int q = 0; q < kSlotsSecond; q += 2, w += zs) *w = make_double2(v[q], v[q + 1]);
-            }
-        } else {
-            Dir3 r[3];
-            zone_dirs<false, Bk>(bz.zc, cur, r);
-            if (keep) {
-                const double v[kSlotsFirst] = {r[0].d1, r[1].d1, r[2].d1,
-                                               r[0].ko + r[1].ko + r[2].ko};
-#pragma unroll
-                for (int q = 0; q < kSlotsFirst; q += 2, w += zs) *w = make_double2(v[q], v[q + 1]);
-            }
-        }
-    }
 }
 
 // One thread per zone, kEqThreads zones of a brick per CTA (a brick of NZ
@@ -187,35 +55,27 @@ deriv_kernel(ConstVars u, const BssnBlockDesc* __restrict__ blocks,
 // g.gx > 0: only zones owning their node run and write the right-hand side
 // at the node index of the zipped grid; the variables are read there too
 // (zip_in, direct form) or at the padded index.
-template <int BX, int BY, int BZ>
+// bx, by, nz: rows and zones of a brick in the scratch.
 __global__ void __launch_bounds__(kEqThreads, 2)
 eq_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
           const BrickTask* __restrict__ tasks, const double* __restrict__ S, int64_t zs,
-          ZipGrid g, int zip_in) {
-    using Bk = Brick<BX, BY, BZ>;
-    constexpr int PARTS = (Bk::NZ + kEqThreads - 1) / kEqThreads;
+          ZipGrid g, int zip_in, int bx, int by, int nz) {
+    const int parts = (nz + kEqThreads - 1) / kEqThreads;
     extern __shared__ __align__(16) double ring[];  // [kRingPairs][T][2] | vals [NVARS][T]
     const int tid = threadIdx.x;
-    const int task = blockIdx.x / PARTS;
+    const int task = blockIdx.x / parts;
     const BrickTask tk = tasks[task];
     const BssnBlockDesc blk = blocks[tk.blk];
     const int o[3] = {tk.o[0], tk.o[1], tk.o[2]};
     // the zones that run: the brick's extent, or on the zipped grid only the
-    // zones owning their node (a brick on a block's upper face loses its last
-    // layer there unless the face lies on the grid's upper boundary); the
-    // threads are packed onto them, so no lane idles on a skipped zone
-    int ex[3] = {tk.e[0], tk.e[1], tk.e[2]};
-    if (g.gx) {
-        const int n = blk.sz - 2 * PW;
-        const int gd[3] = {g.gx, g.gy, g.gz};
-#pragma unroll
-        for (int d = 0; d < 3; d++)
-            if (o[d] + ex[d] == n && blk.g0[d] + n - 1 != gd[d] - 1) ex[d]--;
-    }
-    const int j = (blockIdx.x % PARTS) * kEqThreads + tid;  // the thread's zone among them
+    // zones owning their node; the threads are packed onto them, so no lane
+    // idles on a skipped zone
+    int ex[3];
+    owned_extent(blk, tk, g, false, ex);
+    const int j = (blockIdx.x % parts) * kEqThreads + tid;  // the thread's zone among them
     if (j >= ex[0] * ex[1] * ex[2]) return;
     const int r0 = j % ex[0], r1 = (j / ex[0]) % ex[1], r2 = j / (ex[0] * ex[1]);
-    const int l = r0 + BX * (r1 + BY * r2);  // zone index in the brick (scratch position)
+    const int l = r0 + bx * (r1 + by * r2);  // zone index in the brick (scratch position)
     const int za0 = o[0] + PW + r0, za1 = o[1] + PW + r1, za2 = o[2] + PW + r2;
     const int64_t pidx = blk.offset + za0 + (int64_t)blk.sz * (za1 + (int64_t)blk.sz * za2);
     int64_t node = pidx;
@@ -223,20 +83,19 @@ eq_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
         node = (blk.g0[0] + za0 - PW) +
                (int64_t)g.gx * ((blk.g0[1] + za1 - PW) + (int64_t)g.gy * (blk.g0[2] + za2 - PW));
     const int64_t in_idx = zip_in ? node : pidx;
-    const double2* in = reinterpret_cast<const double2*>(S) + (int64_t)task * Bk::NZ + l;
+    const double2* in = reinterpret_cast<const double2*>(S) + (int64_t)task * nz + l;
     double2* col = reinterpret_cast<double2*>(ring) + tid;   // this thread's ring column
-    double* vals = ring + kRingSlots * kEqThreads + tid;  // [NVARS][kEqThreads]
+    double* vals = ring + 2 * kRingPairs * kEqThreads + tid;  // [NVARS][kEqThreads]
     // the zone's 24 variables first, as their own commit group
 #pragma unroll
     for (int v = 0; v < NVARS; v++) cp_async8(vals + v * kEqThreads, A.u.p[v] + in_idx);
     cp_async_commit();
-    // slot pair P of the zone lives in ring row P % kRingPairs (slot bases
-    // and counts are even, so a variable's slots are whole pairs)
+    // pair P of the zone lives in ring row P % kRingPairs
     auto issue = [&](int step) {
         if (step < NVARS) {
-            const int b = slot_base(step) / 2, n = slot_len(step) / 2;
+            const int b = pair_base(step), n = stage_second(step) ? kPairsSecond : kPairsFirst;
 #pragma unroll
-            for (int q = 0; q < kSlotsSecond / 2; q++)
+            for (int q = 0; q < kPairsSecond; q++)
                 if (q < n) cp_async16(col + ((b + q) % kRingPairs) * kEqThreads, in + (int64_t)(b + q) * zs);
         }
         cp_async_commit();  // empty groups past the last variable keep the count fixed
@@ -249,19 +108,25 @@ eq_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
     auto get = [&](auto tag, double* d1, double* d2, double& ko) {
         constexpr bool SECOND = decltype(tag)::value;
         cp_async_wait_pending<kPrefetchSteps - 1>();
-        const int b = slot_base(step);
-        auto rd = [&](int q) {
-            const double2 p = col[(((b + q) / 2) % kRingPairs) * kEqThreads];
-            return ((b + q) & 1) ? p.y : p.x;
-        };
-#pragma unroll
-        for (int q = 0; q < 3; q++) d1[q] = rd(q);
+        const int b = pair_base(step);
+        auto rd = [&](int q) { return col[((b + q) % kRingPairs) * kEqThreads]; };
+        const double2 p0 = rd(0);  // dx dy
+        d1[0] = p0.x;
+        d1[1] = p0.y;
         if (SECOND) {
-#pragma unroll
-            for (int q = 0; q < 6; q++) d2[q] = rd(3 + q);
-            ko = rd(9);
+            const double2 p1 = rd(1), p2 = rd(2), p3 = rd(3), p4 = rd(4);  // xx yy | dz zz | xz yz | xy ko
+            d1[2] = p2.x;
+            d2[0] = p1.x;
+            d2[1] = p4.x;
+            d2[2] = p3.x;
+            d2[3] = p1.y;
+            d2[4] = p3.y;
+            d2[5] = p2.y;
+            ko = p4.y;
         } else {
-            ko = rd(3);
+            const double2 p1 = rd(1);  // dz ko
+            d1[2] = p1.x;
+            ko = p1.y;
         }
         issue(step + kPrefetchSteps);  // rows of variables consumed before this one
         step++;
@@ -270,35 +135,28 @@ eq_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
     zone_equations(A, blk, za0, za1, za2, get, pv, store);
 }
 
-constexpr size_t eq_smem_bytes() { return sizeof(double) * kEqThreads * (kRingSlots + NVARS); }
+constexpr size_t eq_smem_bytes() { return sizeof(double) * kEqThreads * (2 * kRingPairs + NVARS); }
 
 struct SplitEntry {
-    int nz, threads;
+    int bx, by, v2, g2, v1, g1, threads, iter, hit, plane, dx_plane;
     size_t smem;
-    void (*deriv)(ConstVars, const BssnBlockDesc*, const BrickTask*, double*, int64_t, ZipGrid);
-    void (*deriv_zip)(ConstVars, const BssnBlockDesc*, const BrickTask*, double*, int64_t, ZipGrid);
-    void (*eq)(RhsArgs, const BssnBlockDesc*, const BrickTask*, const double*, int64_t, ZipGrid, int);
+    void (*deriv)(ConstVars, const BssnBlockDesc*, const AxisCoef*, const BrickTask*, double*, int64_t, ZipGrid, int);
+    void (*deriv_zip)(ConstVars, const BssnBlockDesc*, const AxisCoef*, const BrickTask*, double*, int64_t, ZipGrid, int);
 };
 
-template <int BX, int BY, int BZ>
+template <int BX, int BY>
 SplitEntry make_split() {
-    using Bk = Brick<BX, BY, BZ>;
-    return SplitEntry{Bk::NZ, Bk::THREADS, deriv_smem_bytes<Bk>(),
-                      deriv_kernel<BX, BY, BZ, false>, deriv_kernel<BX, BY, BZ, true>,
-                      eq_kernel<BX, BY, BZ>};
+    using Sh = ColShape<BX, BY>;
+    return SplitEntry{BX, BY, Sh::V2, Sh::G2, Sh::V1, Sh::G1, Sh::T, Sh::ITER, Sh::HIT, Sh::PL, Sh::DXP,
+                      Sh::SMEM, column_kernel<Sh, false>, column_kernel<Sh, true>};
 }
 
-// the fused tiles' shapes in their order, then split-only shapes (bricks too
-// large for the fused kernel's 255 registers per zone)
+// brick shapes (columns; every brick has its block's whole height), in the
+// order of the tile table's split tiles (rhs_fused.cu)
 const SplitEntry* split_table(int* count) {
     static const SplitEntry table[] = {
-        make_split<8, 8, 4>(),
-        make_split<7, 7, 4>(),
-        make_split<8, 4, 4>(),
-        make_split<7, 7, 7>(),
-        make_split<8, 8, 8>(),
-        make_split<13, 5, 5>(),
-        make_split<9, 9, 5>(),
+        make_split<8, 8>(),  make_split<7, 7>(),   make_split<8, 4>(),   make_split<13, 5>(),
+        make_split<9, 9>(),  make_split<13, 13>(), make_split<25, 9>(), make_split<49, 10>(),
     };
     *count = (int)(sizeof(table) / sizeof(table[0]));
     return table;
@@ -312,10 +170,82 @@ int split_shape_count() {
     return c;
 }
 
-int split_zone_count(int shape) {
+int split_columns(int shape, int b[2]) {
     int c;
     const SplitEntry* t = split_table(&c);
-    return (shape < 0 || shape >= c) ? 0 : t[shape].nz;
+    if (shape < 0 || shape >= c) return BSSN_EINVAL;
+    b[0] = t[shape].bx;
+    b[1] = t[shape].by;
+    return 0;
+}
+
+int split_threads(int shape) {
+    int c;
+    const SplitEntry* t = split_table(&c);
+    return (shape < 0 || shape >= c) ? 0 : t[shape].threads;
+}
+
+size_t split_smem(int shape) {
+    int c;
+    const SplitEntry* t = split_table(&c);
+    return (shape < 0 || shape >= c) ? 0 : t[shape].smem;
+}
+
+// Host replay of column_march's shared-memory indexing: every brick the
+// splitter makes of every block side the shape takes, with and without the
+// layers another block owns, with every face of the block physical or none.
+// Returns the number of variable groups that do not fit the CTA's threads and
+// buffers, of taps outside the staged planes and of places outside the ring
+// slots, the d/dx planes or the brick's scratch.
+long split_selfcheck(int shape) {
+    int c;
+    const SplitEntry* tab = split_table(&c);
+    if (shape < 0 || shape >= c) return -1;
+    const SplitEntry& t = tab[shape];
+    const int B[2] = {t.bx, t.by}, TX = t.bx + 2 * PW, T = t.threads;
+    long bad = 0;
+    if (t.v2 * t.g2 < kSecondVars || t.v1 * t.g1 < kFirstVars) bad++;
+    auto case_of = [](int a, int s, int faces) {  // -1: centred
+        if (!faces) return -1;
+        return a <= 5 ? a - 3 : a >= s - 6 ? a - (s - 9) : -1;
+    };
+    for (int s : {13, 19, 31, 55})
+        for (int own = 0; own < 2; own++)
+            for (int faces = 0; faces < 2; faces++) {
+                const int n = s - 2 * PW;
+                const int nb[2] = {(n + B[0] - 1) / B[0], (n + B[1] - 1) / B[1]};
+                for (int q = 0; q < nb[0] * nb[1]; q++) {
+                    int o[2], e[2];
+                    const int qq[2] = {q % nb[0], q / nb[0]};
+                    for (int d = 0; d < 2; d++) {
+                        split1(n, B[d], qq[d], o[d], e[d]);
+                        if (e[d] < 3) bad++;  // a closure reads five points inward
+                        if (own && !faces && o[d] + e[d] == n) e[d]--;
+                        if (e[d] < 1 || e[d] > B[d]) bad++;
+                    }
+                    const int sx = e[0] + 2 * PW, sy = e[1] + 2 * PW, cols = e[0] * e[1];
+                    for (int kind = 0; kind < 2; kind++) {
+                        const int nv = kind ? t.v1 : t.v2;
+                        const int ring = kColRing * nv * t.plane;
+                        const int rings = kind ? ring : ring + kColRing * nv * (t.dx_plane + t.bx * t.by);
+                        if (nv * cols > T || nv * sx * sy > t.iter * T) bad++;
+                        if (!kind && nv * 2 * PW * e[0] > t.hit * T) bad++;
+                        if (rings > (int)(t.smem / sizeof(double))) bad++;
+                    }
+                    // taps of a column along x and y stay in the staged plane
+                    for (int d = 0; d < 2; d++)
+                        for (int i = 0; i < e[d]; i++) {
+                            const int a = o[d] + PW + i, cs = case_of(a, s, faces);
+                            const int lo = cs < 0 ? i : (cs < 3 ? 3 : s - 9) - o[d];
+                            const int hi = cs < 0 ? i + 2 * PW : lo + 5;
+                            if (lo < 0 || hi >= e[d] + 2 * PW) bad++;
+                        }
+                    if ((sy - 1) * TX + sx - 1 >= t.plane) bad++;
+                    if ((sy - 1) * t.bx + e[0] - 1 >= t.dx_plane) bad++;
+                    if (e[0] - 1 + t.bx * (e[1] - 1 + t.by * (n - 1)) >= t.bx * t.by * n) bad++;
+                }
+            }
+    return bad;
 }
 
 int prepare_split(int shape) {
@@ -324,38 +254,39 @@ int prepare_split(int shape) {
     if (shape < 0 || shape >= c) return BSSN_EINVAL;
     int st = set_smem_limit((const void*)t[shape].deriv, (int)t[shape].smem);
     if (!st) st = set_smem_limit((const void*)t[shape].deriv_zip, (int)t[shape].smem);
-    if (!st) st = set_smem_limit((const void*)t[shape].eq, (int)eq_smem_bytes());
+    if (!st) st = set_smem_limit((const void*)eq_kernel, (int)eq_smem_bytes());
     return st;
 }
 
 int launch_rhs_split(int shape, const RhsArgs& A, const BssnBlockDesc* blocks_dev,
                      const BrickTask* tasks_dev, int ntasks, double* scratch,
                      int64_t scratch_zones, cudaStream_t s, KernelTimer* tm,
-                     const int32_t* zip_grid, bool zip_in) {
+                     const int32_t* zip_grid, bool zip_in, int side) {
     int c;
     const SplitEntry* tab = split_table(&c);
-    if (shape < 0 || shape >= c) return BSSN_EINVAL;
+    if (shape < 0 || shape >= c || side <= 2 * PW || !A.axis) return BSSN_EINVAL;
     if (ntasks <= 0) return 0;
     const SplitEntry& t = tab[shape];
-    const int64_t chunk = scratch ? scratch_zones / t.nz : 0;
+    const int nz = t.bx * t.by * (side - 2 * PW);  // zones of a brick in the scratch
+    const int64_t chunk = scratch ? scratch_zones / nz : 0;
     if (chunk <= 0) return BSSN_EINVAL;
     int st = prepare_split(shape);
     if (st) return st;
     const ZipGrid g = zip_grid ? ZipGrid{zip_grid[0], zip_grid[1], zip_grid[2]} : ZipGrid{0, 0, 0};
     zip_in = zip_in && zip_grid;
-    const int64_t zs = chunk * t.nz;  // slot stride
+    const int64_t zs = chunk * nz;  // slot stride
     for (int64_t c0 = 0; c0 < ntasks; c0 += chunk) {
         const int n = (int)(ntasks - c0 < chunk ? ntasks - c0 : chunk);
         if (tm && (st = tm->start(KernelTimer::DERIV, s))) return st;
-        (zip_in ? t.deriv_zip : t.deriv)<<<n, t.threads, t.smem, s>>>(A.u, blocks_dev, tasks_dev + c0,
-                                                                      scratch, zs, g);
+        (zip_in ? t.deriv_zip : t.deriv)<<<n * (t.g2 + t.g1), t.threads, t.smem, s>>>(
+            A.u, blocks_dev, A.axis, tasks_dev + c0, scratch, zs, g, nz);
         st = cuda_status(cudaGetLastError());
         if (!st && tm) st = tm->stop(s);
         if (st) return st;
         if (tm && (st = tm->start(KernelTimer::EQ, s))) return st;
-        const int parts = (t.nz + kEqThreads - 1) / kEqThreads;
-        t.eq<<<n * parts, kEqThreads, eq_smem_bytes(), s>>>(A, blocks_dev, tasks_dev + c0, scratch,
-                                                             zs, g, zip_in ? 1 : 0);
+        const int parts = (nz + kEqThreads - 1) / kEqThreads;
+        eq_kernel<<<n * parts, kEqThreads, eq_smem_bytes(), s>>>(A, blocks_dev, tasks_dev + c0, scratch, zs,
+                                                                 g, zip_in ? 1 : 0, t.bx, t.by, nz);
         st = cuda_status(cudaGetLastError());
         if (!st && tm) st = tm->stop(s);
         if (st) return st;

@@ -115,8 +115,9 @@ int64_t bssn_mesh_unzip_size(bssn_mesh mesh);
 /* All blocks of a mesh in one launch.  Replaces bssnRHS(unzipVarsRHS,
  * uZipVars, blkList, numBlocks, t, uZipConstVars) (rhs.cpp:10-73) and the
  * GPU comparator device::bssnrhs3 (cuda/include/bssn_kernels.cuh:1526-1538).
- * tile: -1 = the split 7x7x7 tile; otherwise a tile id in
- * [0, bssn_tile_count()). */
+ * tile: -1 = each block side's default split tile; otherwise a tile id in
+ * [0, bssn_tile_count()) (split tiles wider than a block's interior leave
+ * that side to its default). */
 int bssn_rhs_blocks_f64(bssn_mesh mesh, double* const* rhs_dev,
                         const double* const* u_dev, const BssnParams* params,
                         int tile, bssn_stream_t stream);
@@ -443,12 +444,13 @@ int bssn_rk4_plan_copy_diag_fields(bssn_rk4_plan plan, double* const* dst_dev, i
  * increasing side order, 1e30 for tiles not timed. */
 int bssn_rk4_plan_autotune(bssn_rk4_plan plan, double* const* u_dev, int reps,
                            bssn_stream_t stream, float* times);
-/* The tile the plan runs for block side `side` (the autotuned or pinned
- * one; before either, the split 7x7x7 tile). */
+/* The tile the plan runs for block side `side`: the autotuned or pinned one
+ * where the plan can run it, else the side's default split tile. */
 int bssn_rk4_plan_tile(bssn_rk4_plan plan, int side);
 /* Pin the tile for block side `side` (0: every side; direct plans take one
  * split tile for all sides), as the autotuner would; the next step
- * recaptures its graph.  BSSN_EINVAL for a tile the plan cannot run. */
+ * recaptures its graph.  Sides whose interior is narrower than a split tile's
+ * brick keep their default.  BSSN_EINVAL for a tile the plan cannot run. */
 int bssn_rk4_plan_set_tile(bssn_rk4_plan plan, int side, int tile);
 /* Enforcement violations accumulated since creation (blocking read). */
 int bssn_rk4_plan_violations(bssn_rk4_plan plan, int* count);
@@ -521,8 +523,9 @@ int bssn_halo_unpack_f64(double* const* u_dev, const double* buf_dev,
 /* Number of compiled tiles and their brick shape (bx, by, bz, threads).
  * A tile runs its brick shape either fused (one kernel forms the derivatives
  * in registers and evaluates the equations) or split (a derivative pass
- * writes every zone's derivatives to a mesh-owned scratch of 162 doubles per
- * zone, at most 6 Mi zones, allocated by bssn_rk4_plan_create or by the
+ * marches the brick's bx x by columns through the whole height of the block
+ * and writes every zone's derivatives to a mesh-owned scratch of 162 doubles
+ * per zone, at most 6 Mi zones, allocated by bssn_rk4_plan_create or by the
  * first bssn_rhs_blocks_f64 call with that tile; an equation pass reads them
  * back).  Both give the same result. */
 int bssn_tile_count(void);

@@ -1,0 +1,78 @@
+"""The split right-hand side's derivative pass (columns marched along z) where
+its indexing can go wrong: every block side, with no face, single faces,
+edges and all six faces physical, under every split tile, against the oracle
+on noise around the flat metric; padding beyond physical faces, which the
+reference never reads, holds NaN."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle_lib as ol
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+FLAGS = (0, 1, 2, 4, 8, 16, 32, 21, 42, 63)
+
+
+def _blocks(B, side):
+    """One block per face set, next to each other in memory only."""
+    blocks = (B.BssnBlockDesc * len(FLAGS))()
+    h = 1.0 / 6.0
+    for b, fl in enumerate(FLAGS):
+        blk = blocks[b]
+        blk.offset, blk.sz, blk.bflag = b * ((side ** 3 + 1) // 2 * 2), side, fl
+        for k in range(3):
+            blk.g0[k] = 0
+            blk.ptmin[k] = 0.3 * (b - 4) + 0.1 * k - 3 * h
+            blk.ptmax[k] = blk.ptmin[k] + (side - 1) * h
+    G = (6 * ((side - 7) // 6) + 1,) * 3
+    return B.MeshSpec(blocks, len(FLAGS), G, h, 0.0, np.full(len(FLAGS), side, dtype=np.int32))
+
+
+@pytest.mark.parametrize("side", [13, 19, 31, 55])
+def test_every_face_set_and_split_tile(side):
+    import bssn_b200 as B
+    spec = _blocks(B, side)
+    rng = np.random.default_rng(side)
+    U = np.zeros((24, spec.n_unzip))
+    U[[0, 1, 12, 15, 17]] = 1.0
+    U += 1e-3 * rng.uniform(-1, 1, U.shape)
+    ref = np.zeros_like(U)
+    for b in range(spec.nblocks):
+        blk = spec.blocks[b]
+        n = side ** 3
+        v = np.ascontiguousarray(U[:, int(blk.offset):int(blk.offset) + n])
+        r = ol.oracle().bssnrhs(v, 0, np.array(list(blk.ptmin)), np.array(list(blk.ptmax)), side, int(blk.bflag),
+                                ol.params())
+        ref[:, int(blk.offset):int(blk.offset) + n] = np.asarray(r).reshape(24, n)
+        cube = v.reshape(24, side, side, side)
+        for axis in range(3):  # x is the last axis
+            ax = 3 - axis
+            if blk.bflag >> (2 * axis) & 1:
+                cube[(slice(None),) * ax + (slice(0, 3),)] = np.nan
+            if blk.bflag >> (2 * axis + 1) & 1:
+                cube[(slice(None),) * ax + (slice(side - 3, side),)] = np.nan
+        U[:, int(blk.offset):int(blk.offset) + n] = v
+    mask = np.zeros(spec.n_unzip, dtype=bool)
+    for b in range(spec.nblocks):
+        m = np.zeros((side,) * 3, dtype=bool)
+        m[3:-3, 3:-3, 3:-3] = True
+        off = int(spec.blocks[b].offset)
+        mask[off:off + side ** 3] = m.reshape(-1)
+    mesh = B.Mesh(spec)
+    dU = torch.from_numpy(U).cuda()
+    split = [t for t in range(len(B.tiles())) if B.tile_mode(t) == 1]
+    first = None
+    for t in [-1] + split:
+        dR = torch.zeros_like(dU)
+        mesh.rhs(dR, dU, B.default_params(), tile=t)
+        torch.cuda.synchronize()
+        got = dR.cpu().numpy()[:, mask]
+        # the bound of every right-hand-side test: 1e-12 of the variable's largest value
+        err = ol.rel_err(ref[:, mask], got)
+        assert err.max() <= 1e-12, (t, err.max(), int(err.argmax()))
+        # every tile applies the same stencils and the same equations
+        first = got if first is None else first
+        assert np.array_equal(first, got), t
