@@ -23,7 +23,11 @@
 namespace bssn {
 namespace {
 
-constexpr int CHUNK = 1024;
+// Points per CTA of the ghost fill and the gather back, one a thread.  Runs of
+// 1,024 left one CTA of 64-register threads per SM, and the last run of a 13^3
+// block (149 of 1,024 threads) a seventh full: ghost fill of 512 such blocks
+// 68 us, in runs of 256 51.
+constexpr int CHUNK = 256;
 
 // Ghost fill.  One CTA per chunk of consecutive padded points of one block:
 // consecutive threads read consecutive nodes of a grid row and write
