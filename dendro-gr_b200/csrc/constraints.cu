@@ -7,11 +7,18 @@
 // and the norm sqrt(sum c^2 / N) over the zipped nodes outside the puncture
 // radii (BSSN_GR/include/grUtils.tcc:36-134).
 //
-// A diagnostic, run every few steps, so it favours simplicity: one thread per
-// owned interior node, derivatives read straight from the padded block in
-// global memory (cached), with the bit-exact stencils of stencil_exact.cuh;
-// mixed derivatives are first derivatives of on-the-fly first derivatives,
-// in the reference's order (d/dy(d/dx), d/dz(d/dx), d/dz(d/dy)).
+// The algebra at one node is one function over where the node's derivatives
+// come from.  Single-level meshes run the split right-hand side's derivative
+// pass (rhs_columns.cuh) on the seventeen variables the constraints
+// differentiate, chunk by chunk into the mesh's scratch, and read them back
+// per zone.  Level meshes, and calls that cannot have the scratch, read the
+// stencils straight from the padded block in global memory (cached) with the
+// bit-exact stencils of stencil_exact.cuh; mixed derivatives are then first
+// derivatives of on-the-fly first derivatives, in the reference's order
+// (d/dy(d/dx), d/dz(d/dx), d/dz(d/dy)): seven times the loads and arithmetic
+// of the derivative pass for every mixed derivative, at 255 registers.
+// Constraints and psi4 of 227 k nodes in 1,000 blocks of 13^3: 3.81 ms that
+// way, 0.5 ms through the derivative pass.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,6 +27,7 @@
 #include "constraints.h"
 #include "kernels.cuh"
 #include "mesh.h"
+#include "rhs_columns.cuh"
 #include "stencil_exact.cuh"
 
 namespace bssn {
@@ -91,6 +99,67 @@ __device__ __forceinline__ double Dmix(const Blk& b, const double* u, int inner,
                b.bflag & (1u << (2 * outer + 1)), b.cf[outer]);
 }
 
+// Derivatives at a node from the padded block's values.
+struct BlockDerivs {
+    const ConstVars& P;
+    const BssnBlockDesc& bd;
+    Blk b;
+    __device__ BlockDerivs(const ConstVars& P_, const BssnBlockDesc& bd_, const int a[3]) : P(P_), bd(bd_) {
+        b.s = bd.sz;
+        b.bflag = bd.bflag;
+        for (int d = 0; d < 3; d++) {
+            b.a[d] = a[d];
+            b.cf[d] = axis_coef((bd.ptmax[d] - bd.ptmin[d]) / (bd.sz - 1));
+        }
+    }
+    __device__ void first(int v, double d1[3]) const {
+        for (int d = 0; d < 3; d++) d1[d] = D1(b, P.p[v] + bd.offset, d);
+    }
+    __device__ void second(int v, double d1[3], double d2[6]) const {
+        const double* u = P.p[v] + bd.offset;
+        first(v, d1);
+        d2[0] = D2(b, u, 0);
+        d2[3] = D2(b, u, 1);
+        d2[5] = D2(b, u, 2);
+        d2[1] = Dmix(b, u, 0, 1);
+        d2[2] = Dmix(b, u, 0, 2);
+        d2[4] = Dmix(b, u, 1, 2);
+    }
+};
+
+// ... and from the derivative pass's scratch (its pairs of the variable at
+// stage_order position `step`, zs pairs apart).
+struct ScratchDerivs {
+    const double2* w;
+    int64_t zs;
+    __device__ static constexpr int step_of(int v) {
+        return v >= U_SYMAT0 ? 14 + v - U_SYMAT0 : v >= U_SYMGT0 ? 3 + v - U_SYMGT0 : v == U_CHI ? 12
+             : v == U_K ? 20 : 9 + v - U_GT0;
+    }
+    __device__ void first(int v, double d1[3]) const {  // a variable without second derivatives
+        const double2* p = w + (int64_t)pair_base(step_of(v)) * zs;
+        const double2 a = __ldg(p), b = __ldg(p + zs);  // dx dy | dz ko
+        d1[0] = a.x;
+        d1[1] = a.y;
+        d1[2] = b.x;
+    }
+    __device__ void second(int v, double d1[3], double d2[6]) const {
+        const double2* p = w + (int64_t)pair_base(step_of(v)) * zs;
+        const double2 a = __ldg(p), b = __ldg(p + zs), c = __ldg(p + 2 * zs), d = __ldg(p + 3 * zs),
+                      e = __ldg(p + 4 * zs);  // dx dy | xx yy | dz zz | xz yz | xy ko
+        d1[0] = a.x;
+        d1[1] = a.y;
+        d1[2] = c.x;
+        d2[0] = b.x;
+        d2[1] = e.x;
+        d2[2] = d.x;
+        d2[3] = b.y;
+        d2[4] = d.y;
+        d2[5] = c.y;
+    }
+};
+
+// The constraints at padded point `a` of a block, written at `node`.
 // PSI4: also the Weyl scalar psi4 into out.p[4] (real) and out.p[5]
 // (imaginary) -- CodeGen/constraints.py:45-244, per point as
 // BSSN_GR/src/physcon.cpp:72-85 (coordinates ptmin + a h of the padded
@@ -100,24 +169,11 @@ __device__ __forceinline__ double Dmix(const Blk& b, const double* u, int inner,
 // psi4 = -(P1 + P2 - P3 - P4) real, P1 + P2 - P3 - P4 imaginary, with
 // P1 = R_ij M^ij, P2 = A_temp At_ij M^ij, P3 = (MR_ij Uu_ij - NR_ij Vv_ij)/chi
 // and P4 the (At r) and d chi products of the definition.
-template <bool PSI4>
-__device__ void constraints_node(const ConstVars& P, const MutVars& out, const BssnBlockDesc& bd,
-                                 int64_t q, int gx, int gy, int gz, int64_t node_at = -1) {
-    const int s = bd.sz, N = s - 6;
-    const int i = (int)(q % N), j = (int)((q / N) % N), k = (int)(q / ((int64_t)N * N));
-    const int64_t x = bd.g0[0] + i, y = bd.g0[1] + j, z = bd.g0[2] + k;
-    const bool own = (i < N - 1 || x == gx - 1) && (j < N - 1 || y == gy - 1) &&
-                     (k < N - 1 || z == gz - 1);
-    if (node_at < 0 && !own) return;
-    Blk b;
-    b.s = s;
-    b.a[0] = i + 3;
-    b.a[1] = j + 3;
-    b.a[2] = k + 3;
-    b.bflag = bd.bflag;
-    for (int d = 0; d < 3; d++) b.cf[d] = axis_coef((bd.ptmax[d] - bd.ptmin[d]) / (s - 1));
-    const int64_t pidx = bd.offset + b.a[0] + (int64_t)s * (b.a[1] + (int64_t)s * b.a[2]);
-    auto V = [&](int v) { return P.p[v] + bd.offset; };
+template <bool PSI4, class Derivs>
+__device__ __forceinline__ void constraints_point(const ConstVars& P, const MutVars& out, const BssnBlockDesc& bd,
+                                                  const int at[3], int64_t node, const Derivs& dv) {
+    const int s = bd.sz;
+    const int64_t pidx = bd.offset + at[0] + (int64_t)s * (at[1] + (int64_t)s * at[2]);
     auto pv = [&](int v) { return P.p[v][pidx]; };
 
     double g[6], ig[6];
@@ -139,15 +195,8 @@ __device__ void constraints_node(const ConstVars& P, const MutVars& out, const B
     // metric derivatives and ig^lm d_l d_m g_ij
     double dg[6][3], Lg[6];
     for (int c = 0; c < 6; c++) {
-        const double* u = V(U_SYMGT0 + c);
         double d2[6];
-        for (int d = 0; d < 3; d++) dg[c][d] = D1(b, u, d);
-        d2[0] = D2(b, u, 0);
-        d2[3] = D2(b, u, 1);
-        d2[5] = D2(b, u, 2);
-        d2[1] = Dmix(b, u, 0, 1);
-        d2[2] = Dmix(b, u, 0, 2);
-        d2[4] = Dmix(b, u, 1, 2);
+        dv.second(U_SYMGT0 + c, dg[c], d2);
         Lg[c] = ig[0] * d2[0] + ig[3] * d2[3] + ig[5] * d2[5] +
                 2.0 * (ig[1] * d2[1] + ig[2] * d2[2] + ig[4] * d2[4]);
     }
@@ -178,9 +227,8 @@ __device__ void constraints_node(const ConstVars& P, const MutVars& out, const B
         R[c] = rt;
     }
     for (int kk = 0; kk < 3; kk++) {
-        const double* u = V(U_GT0 + kk);
         double dG[3];
-        for (int d = 0; d < 3; d++) dG[d] = D1(b, u, d);
+        dv.first(U_GT0 + kk, dG);
         for (int c = 0; c < 6; c++) {
             const int a = sym_a(c), bb = sym_b(c);
             R[c] += 0.5 * (Gm(kk, a) * dG[bb] + Gm(kk, bb) * dG[a]);
@@ -188,16 +236,7 @@ __device__ void constraints_node(const ConstVars& P, const MutVars& out, const B
     }
     const double chi = pv(U_CHI), K = pv(U_K);
     double dchi[3], ddchi[6];
-    {
-        const double* u = V(U_CHI);
-        for (int d = 0; d < 3; d++) dchi[d] = D1(b, u, d);
-        ddchi[0] = D2(b, u, 0);
-        ddchi[3] = D2(b, u, 1);
-        ddchi[5] = D2(b, u, 2);
-        ddchi[1] = Dmix(b, u, 0, 1);
-        ddchi[2] = Dmix(b, u, 0, 2);
-        ddchi[4] = Dmix(b, u, 1, 2);
-    }
+    dv.second(U_CHI, dchi, ddchi);
     {
         const double ichi = 1.0 / chi;
         double T = 0.0;
@@ -228,13 +267,11 @@ __device__ void constraints_node(const ConstVars& P, const MutVars& out, const B
         ham += w * chi * ig[c] * R[c];
         sqrA += w * A[c] * AUU[c];
     }
-    const int64_t node = node_at >= 0 ? node_at : x + (int64_t)gx * (y + (int64_t)gy * z);
     out.p[0][node] = ham - sqrA + 2.0 / 3.0 * K * K;
     double dK[3];
-    for (int d = 0; d < 3; d++) dK[d] = D1(b, V(U_K), d);
+    dv.first(U_K, dK);
     double dA[6][3];
-    for (int c = 0; c < 6; c++)
-        for (int d = 0; d < 3; d++) dA[c][d] = D1(b, V(U_SYMAT0 + c), d);
+    for (int c = 0; c < 6; c++) dv.first(U_SYMAT0 + c, dA[c]);
     for (int a = 0; a < 3; a++) {
         double m = 0.0;
         for (int bb = 0; bb < 3; bb++)
@@ -253,7 +290,7 @@ __device__ void constraints_node(const ConstVars& P, const MutVars& out, const B
         double crd[3];
         for (int d = 0; d < 3; d++) {
             const double h = (bd.ptmax[d] - bd.ptmin[d]) / (s - 1);
-            crd[d] = __dadd_rn(bd.ptmin[d], __dmul_rn((double)b.a[d], h));
+            crd[d] = __dadd_rn(bd.ptmin[d], __dmul_rn((double)at[d], h));
         }
         if (fabs(crd[0]) <= 1e-7 && fabs(crd[1]) <= 1e-7) {
             out.p[4][node] = 0.0;
@@ -325,6 +362,46 @@ __device__ void constraints_node(const ConstVars& P, const MutVars& out, const B
         out.p[4][node] = -(p1r + Atmp * q2r - ichi * s3r - p4r);
         out.p[5][node] = p1i + Atmp * q2i - ichi * s3i - p4i;
     }
+}
+
+// Zone q of a block from the block's values: written at node_at (>= 0), or at
+// the zone's own node when the block owns it.
+template <bool PSI4>
+__device__ void constraints_node(const ConstVars& P, const MutVars& out, const BssnBlockDesc& bd,
+                                 int64_t q, int gx, int gy, int gz, int64_t node_at = -1) {
+    const int N = bd.sz - 6;
+    const int i = (int)(q % N), j = (int)((q / N) % N), k = (int)(q / ((int64_t)N * N));
+    const int64_t x = bd.g0[0] + i, y = bd.g0[1] + j, z = bd.g0[2] + k;
+    const bool own = (i < N - 1 || x == gx - 1) && (j < N - 1 || y == gy - 1) &&
+                     (k < N - 1 || z == gz - 1);
+    if (node_at < 0 && !own) return;
+    const int at[3] = {i + 3, j + 3, k + 3};
+    const int64_t node = node_at >= 0 ? node_at : x + (int64_t)gx * (y + (int64_t)gy * z);
+    constraints_point<PSI4>(P, out, bd, at, node, BlockDerivs(P, bd, at));
+}
+
+// The zones of a chunk's bricks that own their node, packed onto the threads
+// as in the equation pass, derivatives from the scratch.
+template <bool PSI4>
+__global__ void __launch_bounds__(128) constraints_scratch_kernel(ConstVars P, MutVars out,
+                                                                  const BssnBlockDesc* __restrict__ blocks,
+                                                                  const BrickTask* __restrict__ tasks,
+                                                                  const double* __restrict__ S, int64_t zs,
+                                                                  ZipGrid g, int bx, int by, int nz) {
+    const int parts = (nz + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int task = blockIdx.x / parts;
+    const BrickTask tk = tasks[task];
+    const BssnBlockDesc bd = blocks[tk.blk];
+    int ex[3];
+    owned_extent(bd, tk, g, false, ex);
+    const int j = (blockIdx.x % parts) * blockDim.x + threadIdx.x;
+    if (j >= ex[0] * ex[1] * ex[2]) return;
+    const int r0 = j % ex[0], r1 = (j / ex[0]) % ex[1], r2 = j / (ex[0] * ex[1]);
+    const int at[3] = {tk.o[0] + PW + r0, tk.o[1] + PW + r1, tk.o[2] + PW + r2};
+    const int64_t node = (bd.g0[0] + at[0] - PW) +
+                         (int64_t)g.gx * ((bd.g0[1] + at[1] - PW) + (int64_t)g.gy * (bd.g0[2] + at[2] - PW));
+    const ScratchDerivs dv{reinterpret_cast<const double2*>(S) + (int64_t)task * nz + r0 + bx * (r1 + by * r2), zs};
+    constraints_point<PSI4>(P, out, bd, at, node, dv);
 }
 
 // One CTA per chunk of up to 1024 interior points of a block, 256 threads
@@ -424,21 +501,93 @@ __global__ void __launch_bounds__(256) l2_partial_kernel(ConstVars C, int nc, in
 }
 
 // sums: write the raw sums of squares (out[0..nc-1]) and the node count
-// (out[4]) for a reduction over ranks instead of the norms
-__global__ void l2_final_kernel(const double* partial, int nblocks, int nc, double* norms, bool sums) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// (out[4]) for a reduction over ranks instead of the norms.  One CTA: thread t
+// adds the partials t, t + 256, ... in order, then a tree over the threads, a
+// fixed order whatever the timing (one thread adding all 592 partials in
+// turn took 107 us, this 4).
+__global__ void __launch_bounds__(256) l2_final_kernel(const double* __restrict__ partial, int nblocks, int nc,
+                                                       double* norms, bool sums) {
+    __shared__ double red[256][5];
     double s[5] = {0, 0, 0, 0, 0};
-    for (int b = 0; b < nblocks; b++)
+    for (int b = threadIdx.x; b < nblocks; b += 256)
         for (int c = 0; c < 5; c++) s[c] += partial[b * 5 + c];
+    for (int c = 0; c < 5; c++) red[threadIdx.x][c] = s[c];
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w)
+            for (int c = 0; c < 5; c++) red[threadIdx.x][c] += red[threadIdx.x + w][c];
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    const double* t = red[0];
     if (sums) {
-        for (int c = 0; c < nc; c++) norms[c] = s[c];
-        norms[4] = s[4];
+        for (int c = 0; c < nc; c++) norms[c] = t[c];
+        norms[4] = t[4];
         return;
     }
-    for (int c = 0; c < nc; c++) norms[c] = s[4] > 0 ? sqrt(s[c] / s[4]) : 0.0;
+    for (int c = 0; c < nc; c++) norms[c] = t[4] > 0 ? sqrt(t[c] / t[4]) : 0.0;
 }
 
-int launch_constraints(const MeshState* m, const double* const* P, double* const* out,
+// The variables the constraints differentiate, as stage_order positions: the
+// metric and chi with second derivatives, Gt^i, At and K without.
+static ColVars constraint_vars() {
+    ColVars c = {};
+    for (int q = 0; q < 6; q++) c.second[c.n2++] = 3 + q;
+    c.second[c.n2++] = 12;
+    for (int q = 0; q < 3; q++) c.first[c.n1++] = 9 + q;
+    for (int q = 14; q <= 20; q++) c.first[c.n1++] = q;
+    return c;
+}
+
+// Single-level meshes: the derivative pass and the algebra, chunk by chunk.
+// Returns BSSN_ENOMEM before any launch when the scratch cannot be had (no
+// device memory, or a capture running and none allocated yet).
+static int constraints_split(MeshState* m, const ConstVars& p, const MutVars& o, cudaStream_t s, bool psi4) {
+    const int64_t nn = (int64_t)m->G[0] * m->G[1] * m->G[2];
+    if (nn >= (int64_t(1) << 31)) return BSSN_ENOMEM;  // node indices of the grid arguments are 32-bit
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {  // the legacy stream while another one captures
+        cudaGetLastError();
+        return BSSN_ENOMEM;
+    }
+    // a chunk of a million zones (1.4 GB) is enough when no plan has made the
+    // scratch larger
+    int64_t need = 0;
+    bool known = true;
+    for (int side : m->sides) {
+        const int t = default_split_tile(side);
+        known = known && m->tasks.count(std::make_pair(t, side));
+        if (cap == cudaStreamCaptureStatusNone || known) need = std::max(need, split_need(m, t, side));
+    }
+    need = std::min<int64_t>(need, int64_t(1) << 20);
+    if (cap != cudaStreamCaptureStatusNone && (!known || m->scratch_zones < need)) return BSSN_ENOMEM;
+    int st = mesh_scratch(m, need);
+    if (st) return BSSN_ENOMEM;
+    const ZipGrid g{m->G[0], m->G[1], m->G[2]};
+    const ColVars vars = constraint_vars();
+    for (int side : m->sides) {
+        const int t = default_split_tile(side);
+        const BrickTask* tk;
+        int nt;
+        st = mesh_tasks_side(m, t, side, &tk, &nt);
+        if (st) return st;
+        st = split_chunks(t, side, p, m->d_axis, m->d_blocks, tk, nt, m->d_scratch, m->scratch_zones, s, g, vars,
+                          [&](const BrickTask* tasks, int n, int64_t zs, const int b[2], int nz) {
+                              const int parts = (nz + 127) / 128;
+                              if (psi4)
+                                  constraints_scratch_kernel<true><<<n * parts, 128, 0, s>>>(
+                                      p, o, m->d_blocks, tasks, m->d_scratch, zs, g, b[0], b[1], nz);
+                              else
+                                  constraints_scratch_kernel<false><<<n * parts, 128, 0, s>>>(
+                                      p, o, m->d_blocks, tasks, m->d_scratch, zs, g, b[0], b[1], nz);
+                              return cuda_status(cudaGetLastError());
+                          });
+        if (st) return st;
+    }
+    return 0;
+}
+
+int launch_constraints(MeshState* m, const double* const* P, double* const* out,
                        cudaStream_t s, bool psi4) {
     ConstVars p;
     MutVars o = {};
@@ -455,6 +604,8 @@ int launch_constraints(const MeshState* m, const double* const* P, double* const
             constraints_levels_kernel<false><<<grid, 256, 0, s>>>(p, o, m->d_blocks, nb, m->lv->zip_src, nn);
         return cuda_status(cudaGetLastError());
     }
+    const int st = constraints_split(m, p, o, s, psi4);
+    if (st != BSSN_ENOMEM) return st;
     if (m->n_int_chunks == 0) return 0;
     if (psi4)
         constraints_kernel<true><<<m->n_int_chunks, 256, 0, s>>>(p, o, m->d_blocks, m->d_int_chunks,
@@ -475,7 +626,7 @@ int launch_l2_norms(const MeshState* m, const double* const* C, int nc, const do
     l2_partial_kernel<<<npartial, 256, 0, s>>>(c, nc, n, m->G[0], m->G[1], xmin[0], xmin[1],
                                                xmin[2], h, bh[0], bh[1], bh[2], bh[3], bh[4],
                                                bh[5], radii[0], radii[1], mask, partial);
-    l2_final_kernel<<<1, 32, 0, s>>>(partial, npartial, nc, norms, sums);
+    l2_final_kernel<<<1, 256, 0, s>>>(partial, npartial, nc, norms, sums);
     return cuda_status(cudaGetLastError());
 }
 

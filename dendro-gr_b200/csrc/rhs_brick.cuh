@@ -131,6 +131,70 @@ __device__ __forceinline__ double closure_d1(const double* t, int st, int a, int
     return __dmul_rn(closure_fold(t, st, 0, c), cf.ih12);
 }
 
+// One-sided closures by table: the three zones next to a face read the same
+// six points.  Weights of those points in increasing order and a mask of the
+// points a (kind, case) uses; the dissipation of a lower face is summed from
+// the far point inward, so its weights and mask are stored for that order.
+struct ClosureTables {
+    double c[3][6][6];
+    unsigned mask[3][6];
+};
+__constant__ ClosureTables kClosures = {
+    {{{-25, 48, -36, 16, -3, 0}, {-3, -10, 18, -6, 1, 0}, {1, -8, 0, 8, -1, 0},
+      {0, 1, -8, 0, 8, -1}, {0, -1, 6, -18, 10, 3}, {0, 3, -16, 36, -48, 25}},
+     {{45, -154, 214, -156, 61, -10}, {10, -15, -4, 14, -6, 1}, {-1, 16, -30, 16, -1, 0},
+      {0, -1, 16, -30, 16, -1}, {1, -6, 14, -4, -15, 10}, {-10, 61, -156, 214, -154, 45}},
+     {{0, 0, 1, -3, 3, -1}, {0, 1, -6, 12, -10, 3}, {1, -6, 15, -19, 12, -3},
+      {1, -6, 15, -19, 12, -3}, {0, 1, -6, 12, -10, 3}, {0, 0, 1, -3, 3, -1}}},
+    {{0x1f, 0x1f, 0x1b, 0x36, 0x3e, 0x3e}, {0x3f, 0x3f, 0x1f, 0x3e, 0x3f, 0x3f}, {0x3c, 0x3e, 0x3f, 0x3f, 0x3e, 0x3c}}};
+
+// the CTA's copy, one entry a thread
+__device__ __forceinline__ void fill_closures(ClosureTables& T, int tid) {
+    if (tid < 108) (&T.c[0][0][0])[tid] = (&kClosures.c[0][0][0])[tid];
+    if (tid < 18) (&T.mask[0][0])[tid] = (&kClosures.mask[0][0])[tid];
+}
+
+// The fold of one closure over the six points t[0], t[st], ... (or, rev, the
+// same points backwards): products and sums of the points in use, in order.
+__device__ __forceinline__ double closure_tab(const ClosureTables& T, int kind, int cs, const double* t, int st) {
+    const bool rev = kind == 2 && cs < 3;
+    const unsigned m = T.mask[kind][cs];
+    const double* c = T.c[kind][cs];
+    if (rev) {
+        t += 5 * st;
+        st = -st;
+    }
+    // selects, not branches: the lanes of a warp sit next to different points
+    double r = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+        const double a = __dadd_rn(r, __dmul_rn(c[j], t[j * st]));
+        r = m >> j & 1u ? a : r;
+    }
+    return r;
+}
+
+__device__ __forceinline__ double closure_smr(int cs, const AxisCoef& cf) {
+    return (cs == 0 || cs == 5) ? cf.smr3 : ((cs == 1 || cs == 4) ? cf.smr2 : cf.smr1);
+}
+
+// closure3 / closure_d1 by table; t points at the zone, a is its padded
+// coordinate.
+template <bool SECOND>
+__device__ __forceinline__ void closure3_tab(const ClosureTables& T, const double* t, int st, int a, int s, bool blo,
+                                             const AxisCoef& cf, double& d1, double& d2, double& ko) {
+    const int c = closure_case(a, s, blo);
+    const double* f = t + ((c < 3 ? 3 : s - 9) - a) * st;
+    d1 = __dmul_rn(closure_tab(T, 0, c, f, st), cf.ih12);
+    if (SECOND) d2 = __dmul_rn(closure_tab(T, 1, c, f, st), cf.ih2_12);
+    ko = __ddiv_rn(closure_tab(T, 2, c, f, st), closure_smr(c, cf));
+}
+__device__ __forceinline__ double closure_d1_tab(const ClosureTables& T, const double* t, int st, int a, int s,
+                                                 bool blo, const AxisCoef& cf) {
+    const int c = closure_case(a, s, blo);
+    return __dmul_rn(closure_tab(T, 0, c, t + ((c < 3 ? 3 : s - 9) - a) * st, st), cf.ih12);
+}
+
 __device__ __forceinline__ bool near_face(int a, int s, bool blo, bool bhi) {
     return (blo && a <= 5) || (bhi && a >= s - 6);
 }
@@ -170,6 +234,7 @@ struct ZoneCtx {
     // per-axis stencil factors: the same for every zone of a block, so they
     // live in shared memory (three AxisCoef in registers would take 48)
     const AxisCoef* cf;
+    const ClosureTables* ct = nullptr;  // shared copy (fill_closures), on-chip kernel
     int tc;          // tile index of the zone
     int st[3];       // tile strides
 };
@@ -309,10 +374,6 @@ __device__ __forceinline__ void mixed_pass(const double* tile, double* mxj, doub
 // for blocks of a single-level mesh, the zipped node grid directly (gx > 0:
 // offsets are node indices, points outside the grid are zero -- exactly the
 // values the ghost fill writes there -- marked -2).
-struct ZipGrid {
-    int gx, gy, gz;  // gx == 0: padded input
-};
-
 template <class Bk, bool ZIP>
 struct StagePlan {
     static constexpr int ITER = (Bk::TILE + Bk::THREADS - 1) / Bk::THREADS;
@@ -348,75 +409,19 @@ struct StagePlan {
     }
 };
 
-// The mixed pass over the compile-time extents of the mixed scratch (items
-// outside a ragged brick's region are skipped); output index = item index.
-template <class Bk>
-__device__ __forceinline__ void mixed_pass_fixed(const double* tile, double* mx, const int o[3],
-                                                 const int e[3], int s, unsigned bflag,
-                                                 const AxisCoef cf[3], int tid) {
-    constexpr int BX = Bk::BX, BY = Bk::BY, TX = Bk::TX, TY = Bk::TY;
-    constexpr int MXJ = Bk::MXJ, MXK = Bk::MXK;
-    for (int idx = tid; idx < MXJ + 2 * MXK; idx += Bk::THREADS) {
-        if (idx < MXJ) {  // d/dx on (x brick, y all, z brick)
-            const int i = idx % BX, r = idx / BX, j = r % TY, k = r / TY;
-            if (i < e[0] && j < e[1] + 2 * PW && k < e[2]) {
-                const double* t = tile + (i + PW) + TX * (j + TY * (k + PW));
-                mx[idx] = d1_exact(t, 1, o[0] + PW + i, s, bflag & 1u, bflag & 2u, cf[0]);
-            }
-            continue;
-        }
-        const bool ydir = idx >= MXJ + MXK;
-        const int q = idx - (ydir ? MXJ + MXK : MXJ);
-        const int i = q % BX, r = q / BX, j = r % BY, k = r / BY;
-        if (i < e[0] && j < e[1] && k < e[2] + 2 * PW) {
-            const double* t = tile + (i + PW) + TX * ((j + PW) + TY * k);
-            mx[idx] = ydir ? d1_exact(t, TX, o[1] + PW + j, s, bflag & 4u, bflag & 8u, cf[1])
-                           : d1_exact(t, 1, o[0] + PW + i, s, bflag & 1u, bflag & 2u, cf[0]);
-        }
-    }
-}
-
-// Interior stencils of one direction, computed for every zone whatever its
-// position (the taps of a zone of the brick always lie in the staged tile);
-// zones near a physical face then take the closure instead.  Doing the three
-// directions without branches lets their nine FP64 chains interleave.
-template <bool SECOND>
-__device__ __forceinline__ Dir3 dir_in(const double* t, int st, const AxisCoef& c) {
-    Dir3 r;
-    r.d1 = d1_in(t, st, c);
-    r.d2 = SECOND ? d2_in(t, st, c) : 0.0;
-    r.ko = ko_in(t, st, c);
-    return r;
-}
 __device__ __forceinline__ double d1_fast_in(const double* t, int st, const AxisCoef& c) {
     const double D1 = t[st] - t[-st], D2 = t[2 * st] - t[-2 * st], D3 = t[3 * st] - t[-3 * st];
     return fma(45.0, D1, fma(-9.0, D2, D3)) * c.ih60;
 }
 
-// Gradient, pure second derivatives and summed KO of the tile's variable at
-// the zone (interior stencils, closures as an override in boundary blocks).
-template <bool SECOND, class Bk>
-__device__ __forceinline__ void zone_dirs(const ZoneCtx& z, const double* tile, Dir3 r[3]) {
-    const double* t = tile + z.tc;
-    // compile-time strides: every tap is an immediate offset
-    r[0] = dir_in<SECOND>(t, 1, z.cf[0]);
-    r[1] = dir_in<SECOND>(t, Bk::TX, z.cf[1]);
-    r[2] = dir_in<SECOND>(t, Bk::TX * Bk::TY, z.cf[2]);
-    if (z.bflag) {
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const bool lo = z.bflag & (1u << (2 * d)), hi = z.bflag & (2u << (2 * d));
-            if (near_face(z.a[d], z.s, lo, hi)) r[d] = closure3(t, z.st[d], z.a[d], z.s, lo, z.cf[d], SECOND);
-        }
-    }
-}
-
-// The interior stencils of zone_dirs (d1_in / d2_in / ko_in along x, y, z)
-// advanced one tap at a time across all nine chains: every chain keeps the
-// reference's left-to-right order of rounded products and sums, but the
-// chains' operations alternate, so each tap step offers nine independent
-// FP64 chains to hide latency with few warps per SM.  Closures as in
-// zone_dirs.
+// Gradient, pure second derivatives and KO of the tile's variable at the zone:
+// the interior stencils (d1_in / d2_in / ko_in along x, y, z), computed for
+// every zone whatever its position (the taps of a zone of the brick always lie
+// in the staged tile), advanced one tap at a time across all nine chains:
+// every chain keeps the reference's left-to-right order of rounded products
+// and sums, but the chains' operations alternate, so each tap step offers nine
+// independent FP64 chains to hide latency with few warps per SM.  Zones near a
+// physical face then take the closure instead.
 template <bool SECOND, class Bk>
 __device__ __forceinline__ void zone_dirs_il(const ZoneCtx& z, const double* tile, Dir3 r[3]) {
     const double* t = tile + z.tc;
@@ -482,7 +487,8 @@ __device__ __forceinline__ void zone_dirs_il(const ZoneCtx& z, const double* til
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             const bool lo = z.bflag & (1u << (2 * d)), hi = z.bflag & (2u << (2 * d));
-            if (near_face(z.a[d], z.s, lo, hi)) r[d] = closure3(t, z.st[d], z.a[d], z.s, lo, z.cf[d], SECOND);
+            if (near_face(z.a[d], z.s, lo, hi))
+                closure3_tab<SECOND>(*z.ct, t, z.st[d], z.a[d], z.s, lo, z.cf[d], r[d].d1, r[d].d2, r[d].ko);
         }
     }
 }
@@ -494,7 +500,10 @@ __device__ __forceinline__ void zone_dirs_il(const ZoneCtx& z, const double* til
 template <class Bk>
 __device__ __forceinline__ void mixed_halo_pass(const double* tile, double* mx, const int o[3],
                                                 const int e[3], int s, unsigned bflag,
-                                                const AxisCoef cf[3], int tid) {
+                                                const AxisCoef cf[3], const ClosureTables& T, int tid) {
+    auto first = [&](const double* t, int st, int a, bool lo, bool hi, const AxisCoef& c) {
+        return near_face(a, s, lo, hi) ? closure_d1_tab(T, t, st, a, s, lo, c) : d1_in(t, st, c);
+    };
     constexpr int BX = Bk::BX, BY = Bk::BY, BZ = Bk::BZ, TX = Bk::TX, TY = Bk::TY;
     constexpr int HJ = BX * 2 * PW * BZ, HK = BX * BY * 2 * PW;
     for (int idx = tid; idx < HJ + 2 * HK; idx += Bk::THREADS) {
@@ -503,7 +512,7 @@ __device__ __forceinline__ void mixed_halo_pass(const double* tile, double* mx, 
             const int j = h < PW ? h : e[1] + h;
             if (i < e[0] && k < e[2]) {
                 const double* t = tile + (i + PW) + TX * (j + TY * (k + PW));
-                mx[i + BX * (j + TY * k)] = d1_exact(t, 1, o[0] + PW + i, s, bflag & 1u, bflag & 2u, cf[0]);
+                mx[i + BX * (j + TY * k)] = first(t, 1, o[0] + PW + i, bflag & 1u, bflag & 2u, cf[0]);
             }
             continue;
         }
@@ -515,9 +524,9 @@ __device__ __forceinline__ void mixed_halo_pass(const double* tile, double* mx, 
             const double* t = tile + (i + PW) + TX * ((j + PW) + TY * k);
             const int w = i + BX * (j + BY * k);
             if (ydir)
-                mx[Bk::MXJ + Bk::MXK + w] = d1_exact(t, TX, o[1] + PW + j, s, bflag & 4u, bflag & 8u, cf[1]);
+                mx[Bk::MXJ + Bk::MXK + w] = first(t, TX, o[1] + PW + j, bflag & 4u, bflag & 8u, cf[1]);
             else
-                mx[Bk::MXJ + w] = d1_exact(t, 1, o[0] + PW + i, s, bflag & 1u, bflag & 2u, cf[0]);
+                mx[Bk::MXJ + w] = first(t, 1, o[0] + PW + i, bflag & 1u, bflag & 2u, cf[0]);
         }
     }
     (void)BZ;

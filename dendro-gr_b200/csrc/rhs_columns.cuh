@@ -22,6 +22,16 @@
 // warps of their own, which run a rolled loop with the table-driven
 // one-sided closures and meet the others at the same barriers; next to a
 // physical z face a pass after the march redoes three zones.
+//
+// What bounds it: FP64 and shared-memory issue, and the barrier per plane.  A
+// zone and variable cost about 100 FP64 warp instructions per 32 zones and 23
+// shared loads of a thread's own; the form that this replaces (a cube of brick
+// + halo per variable, one thread per zone, mixed derivatives through a
+// cooperative halo pass, closures by per-term constant tables) issued about
+// 430 instructions with 52 shared loads.  Derivative passes of one RK4 step:
+// 19.8 M zones in 4,108 mixed blocks 58.2 -> 39 ms, a 2,708-block level mesh
+// 9.3 -> 7.2 ms, 512 blocks of 13^3 (176 k zones, 58 % of the blocks on the
+// boundary) 1.09 -> 0.82 ms.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -92,56 +102,9 @@ struct ColShape {
     static_assert(T <= MAXT && SMEM <= 224 * 1024, "a CTA's threads and shared memory");
 };
 
-// One-sided closures by table: the three zones next to a face read the same
-// six points.  Weights of those points in increasing order and a mask of the
-// points a (kind, case) uses; the dissipation of a lower face is summed from
-// the far point inward, so its weights and mask are stored for that order.
-struct ClosureTables {
-    double c[3][6][6];
-    unsigned mask[3][6];
-};
-__constant__ ClosureTables kClosures = {
-    {{{-25, 48, -36, 16, -3, 0}, {-3, -10, 18, -6, 1, 0}, {1, -8, 0, 8, -1, 0},
-      {0, 1, -8, 0, 8, -1}, {0, -1, 6, -18, 10, 3}, {0, 3, -16, 36, -48, 25}},
-     {{45, -154, 214, -156, 61, -10}, {10, -15, -4, 14, -6, 1}, {-1, 16, -30, 16, -1, 0},
-      {0, -1, 16, -30, 16, -1}, {1, -6, 14, -4, -15, 10}, {-10, 61, -156, 214, -154, 45}},
-     {{0, 0, 1, -3, 3, -1}, {0, 1, -6, 12, -10, 3}, {1, -6, 15, -19, 12, -3},
-      {1, -6, 15, -19, 12, -3}, {0, 1, -6, 12, -10, 3}, {0, 0, 1, -3, 3, -1}}},
-    {{0x1f, 0x1f, 0x1b, 0x36, 0x3e, 0x3e}, {0x3f, 0x3f, 0x1f, 0x3e, 0x3f, 0x3f}, {0x3c, 0x3e, 0x3f, 0x3f, 0x3e, 0x3c}}};
-
-// the CTA's copy, one entry a thread
-__device__ __forceinline__ void fill_closures(ClosureTables& T, int tid) {
-    if (tid < 108) (&T.c[0][0][0])[tid] = (&kClosures.c[0][0][0])[tid];
-    if (tid < 18) (&T.mask[0][0])[tid] = (&kClosures.mask[0][0])[tid];
-}
-
 // x / d for 0 <= x < 2^15 (rounded down) from r = 1 / d: x + 1/2 stays at
 // least 1 / (2 d) away from every multiple of d, far more than the rounding.
 __device__ __forceinline__ int div_small(int x, float r) { return (int)(((float)x + 0.5f) * r); }
-
-// The fold of one closure over the six points t[0], t[st], ... (or, rev, the
-// same points backwards): products and sums of the points in use, in order.
-__device__ __forceinline__ double closure_tab(const ClosureTables& T, int kind, int cs, const double* t, int st) {
-    const bool rev = kind == 2 && cs < 3;
-    const unsigned m = T.mask[kind][cs];
-    const double* c = T.c[kind][cs];
-    if (rev) {
-        t += 5 * st;
-        st = -st;
-    }
-    // selects, not branches: the lanes of a warp sit next to different points
-    double r = 0.0;
-#pragma unroll
-    for (int j = 0; j < 6; j++) {
-        const double a = __dadd_rn(r, __dmul_rn(c[j], t[j * st]));
-        r = m >> j & 1u ? a : r;
-    }
-    return r;
-}
-
-__device__ __forceinline__ double closure_smr(int cs, const AxisCoef& cf) {
-    return (cs == 0 || cs == 5) ? cf.smr3 : ((cs == 1 || cs == 4) ? cf.smr2 : cf.smr1);
-}
 
 template <int N>
 __device__ __forceinline__ double fold6(const double (&c)[N], const double (&u)[6], const int (&p)[N]) {
@@ -218,7 +181,7 @@ __device__ __forceinline__ void owned_extent(const BssnBlockDesc& blk, const Bri
 __device__ __forceinline__ void col_barrier() { asm volatile("bar.sync 0;\n" ::: "memory"); }
 
 template <bool SECOND, class Sh, bool ZIP>
-__device__ __forceinline__ void column_march(int group, int nv, const BrickTask& tk, const BssnBlockDesc& blk,
+__device__ __forceinline__ void column_march(const uint8_t* steps, int nv, const BrickTask& tk, const BssnBlockDesc& blk,
                                              const int ex[3], const double* const* src, const AxisCoef* cfs,
                                              const ClosureTables& CT, double* __restrict__ S, int64_t zs,
                                              const ZipGrid& g, double* ring) {
@@ -232,7 +195,7 @@ __device__ __forceinline__ void column_march(int group, int nv, const BrickTask&
     const int s = blk.sz;
     const int o0 = tk.o[0], o1 = tk.o[1];
     const int np = ex[2] + 2 * PW;  // planes staged
-    auto step_of = [&](int v) { return SECOND ? second_step(group * V + v) : first_step(group * V + v); };
+    auto step_of = [&](int v) { return (int)steps[v]; };  // visiting position of the group's v-th variable
 
     // staged points of this thread: source pointer at the first plane and
     // place in a ring slot (-1: none, <= -2: outside the grid, zero)
@@ -318,7 +281,7 @@ __device__ __forceinline__ void column_march(int group, int nv, const BrickTask&
     const int ax = o0 + PW + cx, ay = o1 + PW + cy;  // padded coordinates
     const int toff = v * PL + (cy + PW) * TX + cx + PW;
     const int mx = v * Sh::DXP + (cy + PW) * BX + cx, my = v * COLS + cy * BX + cx;
-    double2* const w0 = reinterpret_cast<double2*>(S) + (int64_t)pair_base(step_of(v)) * zs + (cx + BX * cy);
+    double2* const w0 = reinterpret_cast<double2*>(S) + (int64_t)pair_base(active ? step_of(v) : 0) * zs + (cx + BX * cy);
     // d/dx on the halo rows of the brick's planes
     constexpr int HIT = Sh::HIT;
     int ht[HIT], hd[HIT], ha[HIT];
@@ -568,36 +531,81 @@ __device__ __forceinline__ void column_march(int group, int nv, const BrickTask&
     }
 }
 
+__host__ __device__ constexpr int col_groups(int n, int v) { return (n + v - 1) / v; }
+
+// A block given by value, for launches without a mesh.
+struct SplitOne {
+    BssnBlockDesc blk;
+    AxisCoef axis[3];
+};
+
+// The q-th brick of such a block under bx x by columns.
+__device__ __forceinline__ BrickTask one_brick(int side, int q, int bx, int by) {
+    const int n = side - 2 * PW, nbx = (n + bx - 1) / bx;
+    BrickTask tk;
+    int o, e;
+    tk.blk = 0;
+    split1(n, bx, q % nbx, o, e);
+    tk.o[0] = (int16_t)o;
+    tk.e[0] = (int16_t)e;
+    split1(n, by, q / nbx, o, e);
+    tk.o[1] = (int16_t)o;
+    tk.e[1] = (int16_t)e;
+    tk.o[2] = 0;
+    tk.e[2] = (int16_t)n;
+    return tk;
+}
+
 // One CTA per (brick, group of variables): the groups with second derivatives
 // first.
 template <class Sh, bool ZIP>
-__global__ void __launch_bounds__(Sh::T, Sh::MINB)
-column_kernel(ConstVars u, const BssnBlockDesc* __restrict__ blocks, const AxisCoef* __restrict__ axis,
-              const BrickTask* __restrict__ tasks,
-              double* __restrict__ S, int64_t zs, ZipGrid g, int nz) {
+__device__ __forceinline__ void column_cta(const ConstVars& u, const BrickTask& tk, const BssnBlockDesc& blk,
+                                           const AxisCoef* axis, int task, int group, double* __restrict__ S,
+                                           int64_t zs, const ZipGrid& g, int nz, const ColVars& vars) {
     extern __shared__ __align__(16) double smem[];
     __shared__ const double* src[NVARS];
     __shared__ AxisCoef cfs[3];
     __shared__ ClosureTables CT;
-    constexpr int G = Sh::G2 + Sh::G1;
-    const int task = blockIdx.x / G, group = blockIdx.x % G;
-    const BrickTask tk = tasks[task];
-    const BssnBlockDesc blk = blocks[tk.blk];
+    __shared__ uint8_t steps[Sh::V2 > Sh::V1 ? Sh::V2 : Sh::V1];
+    const int g2 = col_groups(vars.n2, Sh::V2);
+    const int i0 = group < g2 ? group * Sh::V2 : (group - g2) * Sh::V1;  // the group's first variable
+    const int nv = group < g2 ? min(Sh::V2, vars.n2 - i0) : min(Sh::V1, vars.n1 - i0);
     const int tid = threadIdx.x;
     if (tid < NVARS) src[tid] = u.p[stage_order(tid)] + (ZIP ? 0 : blk.offset);
-    if (tid < 24) (&cfs[0].ih60)[tid] = (&axis[3 * (int64_t)tk.blk].ih60)[tid];
+    if (tid < nv) steps[tid] = group < g2 ? vars.second[i0 + tid] : vars.first[i0 + tid];
+    if (tid < 24) (&cfs[0].ih60)[tid] = (&axis[0].ih60)[tid];
     if (blk.bflag & 15u) fill_closures(CT, tid);
     int ex[3];
     owned_extent(blk, tk, g, true, ex);
     __syncthreads();
     double* Sb = S + 2 * (int64_t)task * nz;
-    if (group < Sh::G2) {
-        const int nv = min(Sh::V2, kSecondVars - group * Sh::V2);
-        column_march<true, Sh, ZIP>(group, nv, tk, blk, ex, src, cfs, CT, Sb, zs, g, smem);
-    } else {
-        const int nv = min(Sh::V1, kFirstVars - (group - Sh::G2) * Sh::V1);
-        column_march<false, Sh, ZIP>(group - Sh::G2, nv, tk, blk, ex, src, cfs, CT, Sb, zs, g, smem);
-    }
+    if (group < g2)
+        column_march<true, Sh, ZIP>(steps, nv, tk, blk, ex, src, cfs, CT, Sb, zs, g, smem);
+    else
+        column_march<false, Sh, ZIP>(steps, nv, tk, blk, ex, src, cfs, CT, Sb, zs, g, smem);
+}
+
+template <class Sh, bool ZIP>
+__global__ void __launch_bounds__(Sh::T, Sh::MINB)
+column_kernel(ConstVars u, const BssnBlockDesc* __restrict__ blocks, const AxisCoef* __restrict__ axis,
+              const BrickTask* __restrict__ tasks, double* __restrict__ S, int64_t zs, ZipGrid g, int nz,
+              ColVars vars) {
+    const int groups = col_groups(vars.n2, Sh::V2) + col_groups(vars.n1, Sh::V1);
+    const int task = blockIdx.x / groups;
+    const BrickTask tk = tasks[task];
+    const BssnBlockDesc blk = blocks[tk.blk];
+    column_cta<Sh, ZIP>(u, tk, blk, axis + 3 * (int64_t)tk.blk, task, blockIdx.x % groups, S, zs, g, nz, vars);
+}
+
+// The bricks of one block.
+template <class Sh>
+__global__ void __launch_bounds__(Sh::T, Sh::MINB)
+column_one_kernel(ConstVars u, const __grid_constant__ SplitOne one, double* __restrict__ S, int64_t zs, int nz,
+                  ColVars vars) {
+    const int groups = col_groups(vars.n2, Sh::V2) + col_groups(vars.n1, Sh::V1);
+    const int task = blockIdx.x / groups;
+    const BrickTask tk = one_brick(one.blk.sz, task, Sh::BX, Sh::BY);
+    column_cta<Sh, false>(u, tk, one.blk, one.axis, task, blockIdx.x % groups, S, zs, ZipGrid{0, 0, 0}, nz, vars);
 }
 
 }  // namespace

@@ -360,6 +360,16 @@ int launch_rhs_tasks(int tile, int side, const RhsArgs& A, const BssnBlockDesc* 
     return st;
 }
 
+int split_chunks(int tile, int side, const ConstVars& u, const AxisCoef* axis, const BssnBlockDesc* blocks_dev,
+                 const BrickTask* tasks_dev, int ntasks, double* scratch, int64_t scratch_zones, cudaStream_t s,
+                 const ZipGrid& g, const ColVars& vars, const ChunkWork& after) {
+    int c;
+    const TileEntry* tab = tile_table(&c);
+    if (tile < 0 || tile >= c || tab[tile].mode != 1) return BSSN_EINVAL;
+    return split_shape_chunks(tab[tile].shape, side, u, axis, blocks_dev, tasks_dev, ntasks, scratch, scratch_zones,
+                              s, g, vars, false, nullptr, after);
+}
+
 int bricks_per_block(int tile, int side) {
     int c;
     const TileEntry* tab = tile_table(&c);
@@ -382,6 +392,10 @@ int launch_rhs_single(int tile, const RhsArgs& A, const BssnBlockDesc& blk,
     const TileEntry* tab = tile_table(&c);
     if (tile < 0 || tile >= c) return BSSN_EINVAL;
     if (tab[tile].mode == 2) return launch_rhs_onchip_single(tab[tile].shape, A, blk, s);
+    if (tab[tile].mode == 1) {
+        const int st = launch_rhs_split_single(tab[tile].shape, A, blk, s);
+        if (st != BSSN_ENOMEM) return st;
+    }
     const TileEntry& t = tab[tab[tile].fused];
     int st = prepare(t);
     if (st) return st;

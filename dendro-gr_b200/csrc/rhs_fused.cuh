@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <vector>
 
 #include "bssn_b200.h"
@@ -15,6 +16,18 @@ struct RhsArgs {
     MutVars rhs;
     BssnParams prm;
     const AxisCoef* axis = nullptr;  // stencil factors, three per block of the list's mesh (split tiles)
+};
+
+// The node grid of a single-level mesh (gx == 0: padded blocks).
+struct ZipGrid {
+    int gx, gy, gz;
+};
+
+// Variables a derivative pass covers, as positions in the visiting order
+// (stage_order): n2 with second derivatives, n1 without.
+struct ColVars {
+    uint8_t second[11], first[13];
+    int n2, n1;
 };
 
 // One brick: block index, interior origin and extent per axis.
@@ -105,7 +118,7 @@ int launch_rhs_tasks(int tile, int side, const RhsArgs& A, const BssnBlockDesc* 
 int bricks_per_block(int tile, int side);
 // kernel launches launch_rhs_tasks makes for a task list of ntasks bricks
 int rhs_launch_count(int tile, int ntasks, int64_t scratch_zones, int side);
-// one block; a split tile runs its shape fused
+// one block (a split tile whose scratch cannot be had runs its shape fused)
 int launch_rhs_single(int tile, const RhsArgs& A, const BssnBlockDesc& blk,
                       cudaStream_t s);
 
@@ -118,7 +131,21 @@ int launch_rhs_onchip(int shape, const RhsArgs& A, const BssnBlockDesc* blocks_d
                       const int32_t* zip_grid, bool zip_in);
 int launch_rhs_onchip_single(int shape, const RhsArgs& A, const BssnBlockDesc& blk, cudaStream_t s);
 
+// The derivative pass of a split tile over a task list, a scratch-full of
+// bricks at a time: after(tasks, n, zs, b, nz) enqueues the work on each chunk
+// (its first task and count, the pairs' stride, the columns b and the zones of
+// a brick in the scratch).  u: padded blocks; g: zones that own their node.
+using ChunkWork = std::function<int(const BrickTask*, int, int64_t, const int[2], int)>;
+int split_chunks(int tile, int side, const ConstVars& u, const AxisCoef* axis, const BssnBlockDesc* blocks_dev,
+                 const BrickTask* tasks_dev, int ntasks, double* scratch, int64_t scratch_zones, cudaStream_t s,
+                 const ZipGrid& g, const ColVars& vars, const ChunkWork& after);
 // split path (rhs_split.cu); shape = index among the split shapes
+int split_shape_chunks(int shape, int side, const ConstVars& u, const AxisCoef* axis,
+                       const BssnBlockDesc* blocks_dev, const BrickTask* tasks_dev, int ntasks, double* scratch,
+                       int64_t scratch_zones, cudaStream_t s, const ZipGrid& g, const ColVars& vars, bool zip_in,
+                       KernelTimer* tm, const ChunkWork& after);
+// BSSN_ENOMEM before any launch when its scratch cannot be had
+int launch_rhs_split_single(int shape, const RhsArgs& A, const BssnBlockDesc& blk, cudaStream_t s);
 int split_shape_count();
 int split_columns(int shape, int b[2]);  // columns of a brick
 int split_threads(int shape);    // of the derivative pass

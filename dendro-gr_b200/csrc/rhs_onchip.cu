@@ -70,6 +70,7 @@ onchip_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
     extern __shared__ __align__(16) double smem[];
     __shared__ const double* src[NVARS];
     __shared__ AxisCoef cfs[3];
+    __shared__ ClosureTables CT;
     double* tiles = smem;
     double* mx = smem + kOcBuffers * Bk::TILE;
     double* vals = mx + Bk::MXJ + 2 * Bk::MXK;  // [NVARS][kOcThreads]: the zone's values
@@ -95,10 +96,12 @@ onchip_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
     const int s = blk.sz;
     if (tid < NVARS) src[tid] = A.u.p[stage_order(tid)] + (ZIP ? 0 : blk.offset);
     fill_axis_coefs(cfs, blk, tid);
+    if (blk.bflag) fill_closures(CT, tid);
     // threads past the brick's zones compute on the nearest zone (every
     // index stays in the tile) and store nothing
     const BrickThread<Bk> th(tid, e);
-    const BrickZone<Bk> bz(blk, o, th, cfs);
+    BrickZone<Bk> bz(blk, o, th, cfs);
+    bz.zc.ct = &CT;
     const StagePlan<Bk, ZIP> sp(o, e, s, tid, g, blk.g0);
     const bool zipped = g.gx > 0;
     const bool keep = th.active && (!zipped || oc_owns_node(blk, o, th.t, g));
@@ -145,7 +148,7 @@ onchip_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
                 mx[Bk::MXJ + bz.mxk_off] = r[0].d1;
                 mx[Bk::MXJ + Bk::MXK + bz.mxk_off] = r[1].d1;
             }
-            mixed_halo_pass<Bk>(cur, mx, o, e, s, blk.bflag, bz.zc.cf, tid);
+            mixed_halo_pass<Bk>(cur, mx, o, e, s, blk.bflag, bz.zc.cf, CT, tid);
             __syncthreads();
             const double* mxj = mx + bz.mxj_off;
             const double* mxk = mx + Bk::MXJ + bz.mxk_off;
@@ -156,10 +159,10 @@ onchip_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
             double yz = d1_fast_in(myk, Bk::BX * Bk::BY, zc.cf[2]);
             if (zc.bflag) {
                 if (near_face(zc.a[1], s, zc.bflag & 4u, zc.bflag & 8u))
-                    xy = closure_d1(mxj, bz.mj, zc.a[1], s, zc.bflag & 4u, zc.cf[1]);
+                    xy = closure_d1_tab(CT, mxj, bz.mj, zc.a[1], s, zc.bflag & 4u, zc.cf[1]);
                 if (near_face(zc.a[2], s, zc.bflag & 16u, zc.bflag & 32u)) {
-                    xz = closure_d1(mxk, bz.mk, zc.a[2], s, zc.bflag & 16u, zc.cf[2]);
-                    yz = closure_d1(myk, bz.mk, zc.a[2], s, zc.bflag & 16u, zc.cf[2]);
+                    xz = closure_d1_tab(CT, mxk, bz.mk, zc.a[2], s, zc.bflag & 16u, zc.cf[2]);
+                    yz = closure_d1_tab(CT, myk, bz.mk, zc.a[2], s, zc.bflag & 16u, zc.cf[2]);
                 }
             }
             d1[0] = r[0].d1; d1[1] = r[1].d1; d1[2] = r[2].d1;

@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <map>
+#include <mutex>
 
 #include "bssn_common.cuh"
 #include "rhs_brick.cuh"
@@ -55,24 +57,20 @@ __device__ __forceinline__ void cp_async_wait_pending() {
 // g.gx > 0: only zones owning their node run and write the right-hand side
 // at the node index of the zipped grid; the variables are read there too
 // (zip_in, direct form) or at the padded index.
-// bx, by, nz: rows and zones of a brick in the scratch.
-__global__ void __launch_bounds__(kEqThreads, 2)
-eq_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
-          const BrickTask* __restrict__ tasks, const double* __restrict__ S, int64_t zs,
-          ZipGrid g, int zip_in, int bx, int by, int nz) {
-    const int parts = (nz + kEqThreads - 1) / kEqThreads;
+// bx, by, nz: rows and zones of a brick in the scratch; part: the CTA's
+// kEqThreads zones of the brick.
+__device__ __forceinline__ void eq_cta(const RhsArgs& A, const BrickTask& tk, const BssnBlockDesc& blk, int task,
+                                       int part, const double* __restrict__ S, int64_t zs, const ZipGrid& g,
+                                       int zip_in, int bx, int by, int nz) {
     extern __shared__ __align__(16) double ring[];  // [kRingPairs][T][2] | vals [NVARS][T]
     const int tid = threadIdx.x;
-    const int task = blockIdx.x / parts;
-    const BrickTask tk = tasks[task];
-    const BssnBlockDesc blk = blocks[tk.blk];
     const int o[3] = {tk.o[0], tk.o[1], tk.o[2]};
     // the zones that run: the brick's extent, or on the zipped grid only the
     // zones owning their node; the threads are packed onto them, so no lane
     // idles on a skipped zone
     int ex[3];
     owned_extent(blk, tk, g, false, ex);
-    const int j = (blockIdx.x % parts) * kEqThreads + tid;  // the thread's zone among them
+    const int j = part * kEqThreads + tid;  // the thread's zone among them
     if (j >= ex[0] * ex[1] * ex[2]) return;
     const int r0 = j % ex[0], r1 = (j / ex[0]) % ex[1], r2 = j / (ex[0] * ex[1]);
     const int l = r0 + bx * (r1 + by * r2);  // zone index in the brick (scratch position)
@@ -135,20 +133,42 @@ eq_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
     zone_equations(A, blk, za0, za1, za2, get, pv, store);
 }
 
+__global__ void __launch_bounds__(kEqThreads, 2)
+eq_kernel(RhsArgs A, const BssnBlockDesc* __restrict__ blocks,
+          const BrickTask* __restrict__ tasks, const double* __restrict__ S, int64_t zs,
+          ZipGrid g, int zip_in, int bx, int by, int nz) {
+    const int parts = (nz + kEqThreads - 1) / kEqThreads, task = blockIdx.x / parts;
+    const BrickTask tk = tasks[task];
+    const BssnBlockDesc blk = blocks[tk.blk];
+    eq_cta(A, tk, blk, task, blockIdx.x % parts, S, zs, g, zip_in, bx, by, nz);
+}
+
+// The bricks of one block.
+__global__ void __launch_bounds__(kEqThreads, 2)
+eq_one_kernel(RhsArgs A, const __grid_constant__ SplitOne one, const double* __restrict__ S, int64_t zs, int bx,
+              int by, int nz) {
+    const int parts = (nz + kEqThreads - 1) / kEqThreads, task = blockIdx.x / parts;
+    const BrickTask tk = one_brick(one.blk.sz, task, bx, by);
+    eq_cta(A, tk, one.blk, task, blockIdx.x % parts, S, zs, ZipGrid{0, 0, 0}, 0, bx, by, nz);
+}
+
 constexpr size_t eq_smem_bytes() { return sizeof(double) * kEqThreads * (2 * kRingPairs + NVARS); }
 
 struct SplitEntry {
     int bx, by, v2, g2, v1, g1, threads, iter, hit, plane, dx_plane;
     size_t smem;
-    void (*deriv)(ConstVars, const BssnBlockDesc*, const AxisCoef*, const BrickTask*, double*, int64_t, ZipGrid, int);
-    void (*deriv_zip)(ConstVars, const BssnBlockDesc*, const AxisCoef*, const BrickTask*, double*, int64_t, ZipGrid, int);
+    void (*deriv_one)(ConstVars, SplitOne, double*, int64_t, int, ColVars);
+    void (*deriv)(ConstVars, const BssnBlockDesc*, const AxisCoef*, const BrickTask*, double*, int64_t, ZipGrid, int,
+                  ColVars);
+    void (*deriv_zip)(ConstVars, const BssnBlockDesc*, const AxisCoef*, const BrickTask*, double*, int64_t, ZipGrid, int,
+                  ColVars);
 };
 
 template <int BX, int BY>
 SplitEntry make_split() {
     using Sh = ColShape<BX, BY>;
     return SplitEntry{BX, BY, Sh::V2, Sh::G2, Sh::V1, Sh::G1, Sh::T, Sh::ITER, Sh::HIT, Sh::PL, Sh::DXP,
-                      Sh::SMEM, column_kernel<Sh, false>, column_kernel<Sh, true>};
+                      Sh::SMEM, column_one_kernel<Sh>, column_kernel<Sh, false>, column_kernel<Sh, true>};
 }
 
 // brick shapes (columns; every brick has its block's whole height), in the
@@ -253,45 +273,145 @@ int prepare_split(int shape) {
     const SplitEntry* t = split_table(&c);
     if (shape < 0 || shape >= c) return BSSN_EINVAL;
     int st = set_smem_limit((const void*)t[shape].deriv, (int)t[shape].smem);
+    if (!st) st = set_smem_limit((const void*)t[shape].deriv_one, (int)t[shape].smem);
     if (!st) st = set_smem_limit((const void*)t[shape].deriv_zip, (int)t[shape].smem);
     if (!st) st = set_smem_limit((const void*)eq_kernel, (int)eq_smem_bytes());
+    if (!st) st = set_smem_limit((const void*)eq_one_kernel, (int)eq_smem_bytes());
     return st;
+}
+
+int split_shape_chunks(int shape, int side, const ConstVars& u, const AxisCoef* axis,
+                       const BssnBlockDesc* blocks_dev, const BrickTask* tasks_dev, int ntasks, double* scratch,
+                       int64_t scratch_zones, cudaStream_t s, const ZipGrid& g, const ColVars& vars, bool zip_in,
+                       KernelTimer* tm, const ChunkWork& after) {
+    int c;
+    const SplitEntry* tab = split_table(&c);
+    if (shape < 0 || shape >= c || side <= 2 * PW || !axis) return BSSN_EINVAL;
+    if (ntasks <= 0) return 0;
+    const SplitEntry& t = tab[shape];
+    const int b[2] = {t.bx, t.by};
+    const int nz = t.bx * t.by * (side - 2 * PW);  // zones of a brick in the scratch
+    const int64_t chunk = scratch ? scratch_zones / nz : 0;
+    if (chunk <= 0) return BSSN_EINVAL;
+    int st = prepare_split(shape);
+    if (st) return st;
+    const int groups = col_groups(vars.n2, t.v2) + col_groups(vars.n1, t.v1);
+    const int64_t zs = chunk * nz;  // slot stride
+    for (int64_t c0 = 0; c0 < ntasks; c0 += chunk) {
+        const int n = (int)(ntasks - c0 < chunk ? ntasks - c0 : chunk);
+        if (tm && (st = tm->start(KernelTimer::DERIV, s))) return st;
+        (zip_in ? t.deriv_zip : t.deriv)<<<n * groups, t.threads, t.smem, s>>>(
+            u, blocks_dev, axis, tasks_dev + c0, scratch, zs, g, nz, vars);
+        st = cuda_status(cudaGetLastError());
+        if (!st && tm) st = tm->stop(s);
+        if (!st) st = after(tasks_dev + c0, n, zs, b, nz);
+        if (st) return st;
+    }
+    return 0;
+}
+
+static ColVars all_vars() {
+    ColVars all = {};
+    for (int i = 0; i < kSecondVars; i++) all.second[all.n2++] = (uint8_t)second_step(i);
+    for (int i = 0; i < kFirstVars; i++) all.first[all.n1++] = (uint8_t)first_step(i);
+    return all;
+}
+
+// The scratch of single-block calls comes from one memory pool per device
+// that the library keeps: stream-ordered, so concurrent calls on any streams
+// and threads have their own; at most kOnePoolBytes stay reserved while unused
+// (the largest block's scratch), the rest goes back to the system at the next
+// synchronisation.
+static cudaMemPool_t one_pool() {
+    constexpr uint64_t kOnePoolBytes = uint64_t(160) << 20;
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = pools.find(dev);
+    if (it != pools.end()) return it->second;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kOnePoolBytes;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        pool = nullptr;
+    } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+    }
+    pools[dev] = pool;
+    return pool;
+}
+
+// One block through the two passes: the same kernels, hence the same bits, as
+// a mesh's block.  The fused kernel that served these calls runs a megabyte of
+// straight-line code once and waits for its instructions: 184 us for a 13^3
+// block and 482 for a 55^3 one, here 41 and 117.  BSSN_ENOMEM before any
+// launch when the scratch cannot be had (a stream capture, which would record
+// the allocation, or no memory): the caller then runs the fused kernel.
+int launch_rhs_split_single(int shape, const RhsArgs& A, const BssnBlockDesc& blk, cudaStream_t s) {
+    int c;
+    const SplitEntry* tab = split_table(&c);
+    if (shape < 0 || shape >= c) return BSSN_EINVAL;
+    const SplitEntry& t = tab[shape];
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return BSSN_ENOMEM;
+    }
+    cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? one_pool() : nullptr;
+    if (!pool) return BSSN_ENOMEM;
+    int st = prepare_split(shape);
+    if (st) return st;
+    const int n = blk.sz - 2 * PW;
+    const int bricks = ((n + t.bx - 1) / t.bx) * ((n + t.by - 1) / t.by);
+    const int nz = t.bx * t.by * n;
+    const int64_t zs = (int64_t)bricks * nz;
+    double* scratch = nullptr;
+    if (cudaMallocFromPoolAsync((void**)&scratch, sizeof(double) * kSplitSlots * zs, pool, s) != cudaSuccess) {
+        cudaGetLastError();
+        return BSSN_ENOMEM;
+    }
+    SplitOne one;
+    one.blk = blk;
+    for (int d = 0; d < 3; d++) one.axis[d] = axis_coef((blk.ptmax[d] - blk.ptmin[d]) / (blk.sz - 1));
+    t.deriv_one<<<bricks * (t.g2 + t.g1), t.threads, t.smem, s>>>(A.u, one, scratch, zs, nz, all_vars());
+    st = cuda_status(cudaGetLastError());
+    if (!st) {
+        const int parts = (nz + kEqThreads - 1) / kEqThreads;
+        eq_one_kernel<<<bricks * parts, kEqThreads, eq_smem_bytes(), s>>>(A, one, scratch, zs, t.bx, t.by, nz);
+        st = cuda_status(cudaGetLastError());
+    }
+    const int fr = cuda_status(cudaFreeAsync(scratch, s));
+    return st ? st : fr;
 }
 
 int launch_rhs_split(int shape, const RhsArgs& A, const BssnBlockDesc* blocks_dev,
                      const BrickTask* tasks_dev, int ntasks, double* scratch,
                      int64_t scratch_zones, cudaStream_t s, KernelTimer* tm,
                      const int32_t* zip_grid, bool zip_in, int side) {
-    int c;
-    const SplitEntry* tab = split_table(&c);
-    if (shape < 0 || shape >= c || side <= 2 * PW || !A.axis) return BSSN_EINVAL;
-    if (ntasks <= 0) return 0;
-    const SplitEntry& t = tab[shape];
-    const int nz = t.bx * t.by * (side - 2 * PW);  // zones of a brick in the scratch
-    const int64_t chunk = scratch ? scratch_zones / nz : 0;
-    if (chunk <= 0) return BSSN_EINVAL;
-    int st = prepare_split(shape);
-    if (st) return st;
     const ZipGrid g = zip_grid ? ZipGrid{zip_grid[0], zip_grid[1], zip_grid[2]} : ZipGrid{0, 0, 0};
     zip_in = zip_in && zip_grid;
-    const int64_t zs = chunk * nz;  // slot stride
-    for (int64_t c0 = 0; c0 < ntasks; c0 += chunk) {
-        const int n = (int)(ntasks - c0 < chunk ? ntasks - c0 : chunk);
-        if (tm && (st = tm->start(KernelTimer::DERIV, s))) return st;
-        (zip_in ? t.deriv_zip : t.deriv)<<<n * (t.g2 + t.g1), t.threads, t.smem, s>>>(
-            A.u, blocks_dev, A.axis, tasks_dev + c0, scratch, zs, g, nz);
-        st = cuda_status(cudaGetLastError());
-        if (!st && tm) st = tm->stop(s);
-        if (st) return st;
-        if (tm && (st = tm->start(KernelTimer::EQ, s))) return st;
-        const int parts = (nz + kEqThreads - 1) / kEqThreads;
-        eq_kernel<<<n * parts, kEqThreads, eq_smem_bytes(), s>>>(A, blocks_dev, tasks_dev + c0, scratch, zs,
-                                                                 g, zip_in ? 1 : 0, t.bx, t.by, nz);
-        st = cuda_status(cudaGetLastError());
-        if (!st && tm) st = tm->stop(s);
-        if (st) return st;
-    }
-    return 0;
+    const ColVars all = all_vars();
+    return split_shape_chunks(
+        shape, side, A.u, A.axis, blocks_dev, tasks_dev, ntasks, scratch, scratch_zones, s, g, all, zip_in, tm,
+        [&](const BrickTask* tasks, int n, int64_t zs, const int b[2], int nz) {
+            int st = 0;
+            if (tm && (st = tm->start(KernelTimer::EQ, s))) return st;
+            const int parts = (nz + kEqThreads - 1) / kEqThreads;
+            eq_kernel<<<n * parts, kEqThreads, eq_smem_bytes(), s>>>(A, blocks_dev, tasks, scratch, zs, g,
+                                                                     zip_in ? 1 : 0, b[0], b[1], nz);
+            st = cuda_status(cudaGetLastError());
+            if (!st && tm) st = tm->stop(s);
+            return st;
+        });
 }
 
 }  // namespace bssn

@@ -88,9 +88,12 @@ int bssn_deriv644adv_f64(int dir, double* D_dev, const double* u_dev, double h,
                          unsigned bflag, bssn_stream_t stream);
 
 /* ---------------------------------------------------------------------- */
-/* Fused right-hand side of one block: derivatives, pointwise BSSN
- * equations, Sommerfeld boundary conditions and Kreiss-Oliger dissipation in
- * one kernel; derivatives never leave the chip.
+/* Right-hand side of one block: derivatives, pointwise BSSN equations,
+ * Sommerfeld boundary conditions and Kreiss-Oliger dissipation, the same bits
+ * as the block's in a mesh.  The derivatives pass through scratch from a
+ * stream-ordered memory pool that the library keeps per device (at most 160 MB
+ * stay reserved while unused); under a stream capture, or when no memory is to
+ * be had, one kernel without scratch runs instead.
  * Replaces bssnrhs(unzipVarsRHS, uZipVars, offset, pmin, pmax, sz, bflag,
  * t, uZipConstVars) (BSSN_GR/src/rhs.cpp:80-504, include/rhs.h:32-36); t and
  * the constraint arrays are unused by the standard-gauge equations. */
@@ -176,7 +179,10 @@ int bssn_initial_data_f64(double* const* u_dev, const int32_t G[3],
  * multi-level mesh every zipped node (the level grids back to back) takes
  * the value at the zone that owns it; nodes filled from another level
  * (patch-boundary nodes, coarse nodes under a finer patch) are set to 0, so
- * each physical point carries its value once. */
+ * each physical point carries its value once.  Single-level meshes use the
+ * handle's derivative scratch (allocated here, up to 1.4 GB, when neither a
+ * plan nor bssn_rhs_blocks_f64 has; without it -- no memory, or a stream
+ * capture before it exists -- a slower kernel that needs none runs). */
 int bssn_constraints_f64(bssn_mesh mesh, const double* const* unzip_dev,
                          double* const* cons_dev, bssn_stream_t stream);
 /* The same constraints plus the Weyl scalar psi4 for gravitational-wave

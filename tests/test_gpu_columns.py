@@ -76,3 +76,70 @@ def test_every_face_set_and_split_tile(side):
         # every tile applies the same stencils and the same equations
         first = got if first is None else first
         assert np.array_equal(first, got), t
+
+
+@pytest.mark.parametrize("side", [13, 19, 31, 55])
+def test_single_block_equals_mesh_block(side):
+    """A single-block call runs the mesh's two passes from the library's pool:
+    the same bits as the block in a mesh, on two streams at once, and, where a
+    stream capture forbids the pool, the one-kernel form's (the same stencils
+    and equations: the same bits too)."""
+    import bssn_b200 as B
+    spec = _blocks(B, side)
+    rng = np.random.default_rng(100 + side)
+    U = np.zeros((24, spec.n_unzip))
+    U[[0, 1, 12, 15, 17]] = 1.0
+    U += 1e-3 * rng.uniform(-1, 1, U.shape)
+    dU = torch.from_numpy(U).cuda()
+    prm = B.default_params()
+    mesh = B.Mesh(spec)
+    ref = torch.zeros_like(dU)
+    mesh.rhs(ref, dU, prm)
+    got = torch.zeros_like(dU)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def call(out, b, stream):
+        blk = spec.blocks[b]
+        B.bssnrhs_block(out, dU, int(blk.offset), list(blk.ptmin), list(blk.ptmax), side, int(blk.bflag), prm,
+                        stream=stream)
+
+    for b in range(spec.nblocks):
+        call(got, b, streams[b % 2])
+    torch.cuda.synchronize()
+    assert torch.equal(got, ref)
+    got.zero_()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call(got, 9, torch.cuda.current_stream())
+    g.replay()
+    torch.cuda.synchronize()
+    o = int(spec.blocks[9].offset)
+    assert torch.equal(got[:, o:o + side ** 3], ref[:, o:o + side ** 3])
+
+
+def test_constraints_with_and_without_scratch():
+    """Constraints from the derivative scratch and, captured on a mesh that has
+    none yet, from the padded block directly: the outer stage of the mixed
+    derivatives is rounded differently, 1e-12 of the largest value."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(1, (1, 1, 1), seed=8, xmin=-8.25)
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    out = []
+    for captured in (True, False):
+        mesh = B.Mesh(spec)
+        P = torch.zeros((24, mesh.n_unzip), dtype=torch.float64, device="cuda")
+        mesh.unzip(P, U)
+        cons = torch.zeros((4, spec.n_nodes), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                B.constraints(mesh, cons, P)
+            g.replay()
+        else:
+            B.constraints(mesh, cons, P)
+        torch.cuda.synchronize()
+        out.append(cons.cpu().numpy())
+    assert ol.rel_err(out[0], out[1]).max() <= 1e-12
