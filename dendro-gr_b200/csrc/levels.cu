@@ -391,6 +391,7 @@ int levels_build(const BssnBlockDesc* blocks, int nblocks, const std::vector<Pat
     }
     // owners
     out->zip_src.assign(size_t(out->n_nodes), -1);
+    out->drop.assign(size_t(nblocks), 7);
     for (int p = 0; p < np; p++) {
         const LevelGrid& g = out->grids[p];
         for (int64_t z = 0; z < g.dims[2]; z++)
@@ -429,6 +430,7 @@ int levels_build(const BssnBlockDesc* blocks, int nblocks, const std::vector<Pat
                     for (int d = 0; d < 3; d++) {
                         loc[d] = q[d] - k.g0[d] + 3;
                         if (loc[d] < 3 || loc[d] > k.sz - 4) return BSSN_EINVAL;
+                        if (loc[d] == k.sz - 4) out->drop[size_t(b)] &= uint8_t(~(1u << d));
                     }
                     out->zip_src[size_t(B.node(p, q))] =
                         k.offset + loc[0] + int64_t(k.sz) * (loc[1] + int64_t(k.sz) * loc[2]);
@@ -747,6 +749,7 @@ int levels_upload(const LevelMaps& m, LevelsDev* d) {
         st = BSSN_ENOMEM;
     }
     if (!st) st = upload_vec(m.zip_src, &d->zip_src);
+    if (!st) st = upload_vec(m.drop, &d->drop);
     if (!st) st = upload_vec(m.inject_dst, &d->inject_dst);
     if (!st) st = upload_vec(m.inject_src, &d->inject_src);
     if (!st) st = upload_vec(m.prolong_dst, &d->prolong_dst);
@@ -766,6 +769,7 @@ void levels_free(LevelsDev* d) {
     cudaFree(d->tasks);
     cudaFree(d->it);
     cudaFree(d->zip_src);
+    cudaFree(d->drop);
     cudaFree(d->inject_dst);
     cudaFree(d->inject_src);
     cudaFree(d->prolong_dst);

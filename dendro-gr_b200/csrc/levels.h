@@ -51,6 +51,12 @@ struct LevelMaps {
     int64_t n_padded = 0;
     std::vector<int64_t> unzip_src;              // per padded point
     std::vector<int64_t> zip_src;                // per node: owning zone's padded index or -1
+    // per block, the axes (bits 0..2) along which no zone of its last layer owns
+    // a node: most blocks share that layer's nodes with the next block or take
+    // them from another level.  A plan's right-hand side leaves those layers out
+    // (the stage reads it only at owning zones): equation passes of one step of
+    // the 2,708-block mesh 4.08 -> 3.67 ms.
+    std::vector<uint8_t> drop;
     std::vector<int64_t> inject_dst, inject_src; // coarse node under a finer box <- fine node
     std::vector<int> inject_first;               // per level l >= 1: first entry (size L + 1)
     std::vector<int64_t> prolong_dst, prolong_src; // fine box-boundary node <- coarse source
@@ -81,6 +87,7 @@ struct LevelsDev {
     double* it = nullptr;       // pass results, [var][n_it]
     int64_t n_it = 0;
     int64_t* zip_src = nullptr;
+    uint8_t* drop = nullptr;  // LevelMaps::drop
     int64_t* inject_dst = nullptr;
     int64_t* inject_src = nullptr;
     int64_t* prolong_dst = nullptr;

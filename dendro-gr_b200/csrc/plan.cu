@@ -179,6 +179,7 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
     RhsArgs A;
     A.prm = p->prm;
     A.axis = m->d_axis;
+    A.drop = m->lv ? m->lv->drop : nullptr;
     if (p->direct) {
         double* Rz[NVARS];
         set_ptrs(p->Rz, p->n_nodes, Rz);
@@ -431,6 +432,7 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
     RhsArgs A;
     A.prm = p->prm;
     A.axis = m->d_axis;
+    A.drop = m->lv ? m->lv->drop : nullptr;
     int st = 0;
     if (p->direct) {  // split tiles on the zipped state u
         double* Rz[NVARS];

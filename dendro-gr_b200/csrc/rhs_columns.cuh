@@ -170,6 +170,7 @@ __device__ __forceinline__ void owned_extent(const BssnBlockDesc& blk, const Bri
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         ex[d] = tk.e[d];
+        if (g.drop && tk.o[d] + ex[d] == n && (g.drop[tk.blk] >> d & 1)) ex[d]--;
         if (g.gx && tk.o[d] + ex[d] == n && blk.g0[d] + n - 1 != gd[d] - 1 &&
             !(keep_faces && (blk.bflag & (2u << (2 * d)))))
             ex[d]--;

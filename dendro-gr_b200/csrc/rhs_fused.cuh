@@ -15,12 +15,19 @@ struct RhsArgs {
     ConstVars u;
     MutVars rhs;
     BssnParams prm;
-    const AxisCoef* axis = nullptr;  // stencil factors, three per block of the list's mesh (split tiles)
+    // split tiles: stencil factors, three per block of the list's mesh, and the
+    // layers a padded right-hand side may leave out (ZipGrid)
+    const AxisCoef* axis = nullptr;
+    const uint8_t* drop = nullptr;
 };
 
-// The node grid of a single-level mesh (gx == 0: padded blocks).
+// The node grid of a single-level mesh (gx == 0: padded blocks).  drop
+// (padded right-hand sides of a multi-level mesh): per block, the axes (bits
+// 0..2) along which no zone of its last layer owns a node, so that nothing
+// reads that layer's right-hand side.
 struct ZipGrid {
     int gx, gy, gz;
+    const uint8_t* drop = nullptr;
 };
 
 // Variables a derivative pass covers, as positions in the visiting order

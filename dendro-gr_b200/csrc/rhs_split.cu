@@ -397,7 +397,7 @@ int launch_rhs_split(int shape, const RhsArgs& A, const BssnBlockDesc* blocks_de
                      const BrickTask* tasks_dev, int ntasks, double* scratch,
                      int64_t scratch_zones, cudaStream_t s, KernelTimer* tm,
                      const int32_t* zip_grid, bool zip_in, int side) {
-    const ZipGrid g = zip_grid ? ZipGrid{zip_grid[0], zip_grid[1], zip_grid[2]} : ZipGrid{0, 0, 0};
+    const ZipGrid g = zip_grid ? ZipGrid{zip_grid[0], zip_grid[1], zip_grid[2]} : ZipGrid{0, 0, 0, A.drop};
     zip_in = zip_in && zip_grid;
     const ColVars all = all_vars();
     return split_shape_chunks(
