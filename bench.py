@@ -71,7 +71,7 @@ FLOP_PER_ZONE_STAGE = 6535.0  # 6,439 RHS + 96 RK axpy (per zone, per stage)
 
 SPLIT_SLOTS = 162  # scratch doubles per zone of the split right-hand side
 KIND_NAMES = {"fused": "bssn::rhs_kernel / bssn::onchip_kernel (one-kernel right-hand side)",
-              "deriv": "bssn::deriv_kernel (derivative pass)", "eq": "bssn::eq_kernel (equation pass)"}
+              "deriv": "bssn::column_kernel (derivative pass)", "eq": "bssn::eq_kernel (equation pass)"}
 
 
 def tile_pins(arg):
@@ -107,12 +107,11 @@ def kernel_bytes(sides, chosen, modes):
 
 # DRAM traffic / algorithmic bytes of one launch of each kernel kind, from ncu
 # captures on small workloads (dram__bytes_read.sum + dram__bytes_write.sum
-# over the launch's algorithmic bytes as kernel_bytes counts them): split
-# 7x7x7 on the uniform 512-block workload; the on-chip kernel on the small
-# mixed workload.  Scales a full pass's algorithmic bytes to DRAM traffic.
-# (uniform 512: deriv 257.0 + 143.4 MB against 192 * 2197 * 512 B; eq 249.3 +
-# 17.9 MB against 384 * 343 * 512 B -- the scratch round trip is the excess)
-TRAFFIC_RATIO = {"deriv": 400.4e6 / (192 * 2197 * 512), "eq": 267.2e6 / (384 * 343 * 512)}
+# over the launch's algorithmic bytes as kernel_bytes counts them).  Scales a
+# full pass's algorithmic bytes to DRAM traffic; kinds without a capture of the
+# present kernel report none.  (uniform 512: eq 249.3 + 17.9 MB against
+# 384 * 343 * 512 B -- the scratch round trip is the excess)
+TRAFFIC_RATIO = {"eq": 267.2e6 / (384 * 343 * 512)}
 
 
 def rhs_bytes(sides):
