@@ -172,8 +172,9 @@ bool plan_zipped_rhs(const Plan* p) {
 }
 
 // One right-hand-side pass over every bucket.  Direct plans read the zipped
-// stage state `src` and write Rz; the others read the padded P (filled by
-// the ghost fill) and write R, or Rz when plan_zipped_rhs.
+// stage state `src` and write Rz, as do the others when plan_zipped_rhs (and
+// src is given); else they read the padded P (filled by the ghost fill) and
+// write R, or Rz when plan_zipped_rhs.
 int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src) {
     MeshState* m = p->mesh;
     RhsArgs A;
@@ -238,19 +239,22 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
         }
         return 0;
     }
-    // zipped right-hand side: blocks of kDirectMinSide and more stage from
-    // the zipped stage state `src` (no ghost fill for them)
-    RhsArgs Ad = A;
-    if (zrhs && src)
-        for (int v = 0; v < NVARS; v++) Ad.u.p[v] = src[v];
+    // zipped right-hand side: the tiles are staged from the zipped stage state
+    // `src`, without a ghost fill.  The column pass takes its planes row by row
+    // either way, so the node grid costs it little more than padded blocks,
+    // and the fill (and its padded writes) goes: step of 512 blocks of 13^3
+    // 1.38 -> 1.30 ms, of the 19.8 M-zone mesh 78.6 -> 74.6 ms.  (The cube form
+    // before it gained from padded tiles below 55^3.)
+    const bool direct = zrhs && src;
+    if (direct)
+        for (int v = 0; v < NVARS; v++) A.u.p[v] = src[v];
     for (int side : p->sides) {
         const int t = plan_tile(p, side);
         const BrickTask* tk;
         int nt;
         int st = mesh_tasks_side(m, t, side, &tk, &nt);
-        const bool direct = zrhs && src && side >= kDirectMinSide;
         if (!st)
-            st = launch_rhs_tasks(t, side, direct ? Ad : A, m->d_blocks, tk, nt, s, m->d_scratch,
+            st = launch_rhs_tasks(t, side, A, m->d_blocks, tk, nt, s, m->d_scratch,
                                   m->scratch_zones, tm, zrhs ? m->G : nullptr, direct);
         if (st) return st;
     }
@@ -288,9 +292,7 @@ int plan_enqueue_stage(Plan* p, double* const* u, double dt, int stage, cudaStre
     if (p->direct || plan_zipped_rhs(p)) {
         double* Rz[NVARS];
         set_ptrs(p->Rz, p->n_nodes, Rz);
-        // ghost fill of the blocks staged from padded blocks only
-        int st = p->direct ? 0 : launch_unzip(m, Pp, src, NVARS, s, true);
-        if (!st) st = plan_rhs(p, s, nullptr, src);
+        int st = plan_rhs(p, s, nullptr, src);
         if (!st) st = launch_node_stage(stage, Ip, Ap, u, Rz, p->n_nodes, dt, enf, p->prm.chi_floor,
                                         p->status, s);
         return st;
@@ -587,8 +589,9 @@ int plan_time_kernels(Plan* p, int reps, cudaStream_t s, double out[6]) {
     return st ? st : cuda_status(cudaGetLastError());
 }
 
-// Kernel launches of one RK4 step: per stage the ghost fill, the
-// right-hand-side launches of every bucket, and the zip-stage kernel.
+// Kernel launches of one RK4 step: per stage the ghost fill (none where the
+// right-hand side reads the zipped state), the right-hand-side launches of
+// every bucket, and the stage kernel.
 int plan_launches_per_step(Plan* p) {
     MeshState* m = p->mesh;
     int rhs = 0;
@@ -610,7 +613,7 @@ int plan_launches_per_step(Plan* p) {
             for (size_t k = 0; k + 1 < f->size(); k++) extra += (*f)[k + 1] > (*f)[k] ? 1 : 0;
         return 4 * (rhs + extra);
     }
-    return 4 * (rhs + (p->direct ? 1 : 2));
+    return 4 * (rhs + (p->direct || plan_zipped_rhs(p) ? 1 : 2));
 }
 
 namespace {

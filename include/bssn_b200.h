@@ -388,20 +388,21 @@ int bssn_remesh_element_features_f64(bssn_mesh mesh, const double* const* unzip_
 /* One whole RK4 step as a plan over a mesh (the reference's per-step
  * sequence rkBSSN.cpp:764-860: per stage unzip -> bssnRHS -> zip -> stage
  * update), same result.  The plan owns its scratch buffers, allocated at
- * creation.  Default form: per stage the ghost fill into padded blocks, the
- * right-hand side on them (one launch sequence per block-size bucket with
- * that bucket's tile, or one launch per block with BSSN_PLAN_PER_BLOCK) and
- * the zip fused with the stage algebra; scratch: two padded 24-variable
- * arrays of bssn_mesh_unzip_size doubles and two zipped ones.
+ * creation.  Default form: per stage the right-hand side straight from the
+ * zipped stage state, written zipped (one launch sequence per block-size
+ * bucket with that bucket's tile), and a node-wise stage kernel; with a fused
+ * tile pinned, on multi-level meshes, or with BSSN_PLAN_PER_BLOCK (one launch
+ * per block): the ghost fill into padded blocks, the right-hand side on them
+ * and the zip fused with the stage algebra.  Scratch: two padded 24-variable
+ * arrays of bssn_mesh_unzip_size doubles and three zipped ones.
  * BSSN_PLAN_DIRECT (split tiles; meshes of fewer than 2^31 nodes): every
  * block of the single-level mesh is a box of the node grid, so the right-hand
  * side reads the zipped stage state directly (points outside the grid read
  * as zero, as the ghost fill writes them), writes each node's right-hand
  * side once from the block owning it (the zip's owner rule), and a node-wise
  * kernel applies the stage algebra; scratch: three zipped 24-variable arrays
- * (no padded ones).  Same result; on B200 the padded form is faster (the
- * derivative pass stages contiguous padded rows), the direct form needs far
- * less memory.  With BSSN_PLAN_GRAPH the 4-stage sequence is captured once as
+ * (no padded ones).  Same result and speed; the direct
+ * form needs far less memory.  With BSSN_PLAN_GRAPH the 4-stage sequence is captured once as
  * a CUDA graph and replayed (recaptured when u_dev or dt change).  u_dev (24
  * zipped arrays of G[0]*G[1]*G[2] doubles) is advanced in place. */
 #define BSSN_PLAN_ENFORCE_STAGES 1 /* enforce constraints on stage states */
