@@ -20,10 +20,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <map>
-#include <mutex>
 
 #include "bssn_common.cuh"
+#include "pool.h"
 #include "rhs_brick.cuh"
 #include "rhs_columns.cuh"
 #include "rhs_equations.cuh"
@@ -317,39 +316,6 @@ static ColVars all_vars() {
     return all;
 }
 
-// The scratch of single-block calls comes from one memory pool per device
-// that the library keeps: stream-ordered, so concurrent calls on any streams
-// and threads have their own; at most kOnePoolBytes stay reserved while unused
-// (the largest block's scratch), the rest goes back to the system at the next
-// synchronisation.
-static cudaMemPool_t one_pool() {
-    constexpr uint64_t kOnePoolBytes = uint64_t(160) << 20;
-    static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = pools.find(dev);
-    if (it != pools.end()) return it->second;
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t pool = nullptr;
-    uint64_t keep = kOnePoolBytes;
-    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-        cudaGetLastError();
-        pool = nullptr;
-    } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-        cudaGetLastError();
-    }
-    pools[dev] = pool;
-    return pool;
-}
-
 // One block through the two passes: the same kernels, hence the same bits, as
 // a mesh's block.  The fused kernel that served these calls runs a megabyte of
 // straight-line code once and waits for its instructions: 184 us for a 13^3
@@ -361,13 +327,6 @@ int launch_rhs_split_single(int shape, const RhsArgs& A, const BssnBlockDesc& bl
     const SplitEntry* tab = split_table(&c);
     if (shape < 0 || shape >= c) return BSSN_EINVAL;
     const SplitEntry& t = tab[shape];
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
-        cudaGetLastError();
-        return BSSN_ENOMEM;
-    }
-    cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? one_pool() : nullptr;
-    if (!pool) return BSSN_ENOMEM;
     int st = prepare_split(shape);
     if (st) return st;
     const int n = blk.sz - 2 * PW;
@@ -375,10 +334,8 @@ int launch_rhs_split_single(int shape, const RhsArgs& A, const BssnBlockDesc& bl
     const int nz = t.bx * t.by * n;
     const int64_t zs = (int64_t)bricks * nz;
     double* scratch = nullptr;
-    if (cudaMallocFromPoolAsync((void**)&scratch, sizeof(double) * kSplitSlots * zs, pool, s) != cudaSuccess) {
-        cudaGetLastError();
-        return BSSN_ENOMEM;
-    }
+    st = pool_alloc((void**)&scratch, sizeof(double) * kSplitSlots * zs, s);
+    if (st) return st;
     SplitOne one;
     one.blk = blk;
     for (int d = 0; d < 3; d++) one.axis[d] = axis_coef((blk.ptmax[d] - blk.ptmin[d]) / (blk.sz - 1));
@@ -389,7 +346,7 @@ int launch_rhs_split_single(int shape, const RhsArgs& A, const BssnBlockDesc& bl
         eq_one_kernel<<<bricks * parts, kEqThreads, eq_smem_bytes(), s>>>(A, one, scratch, zs, t.bx, t.by, nz);
         st = cuda_status(cudaGetLastError());
     }
-    const int fr = cuda_status(cudaFreeAsync(scratch, s));
+    const int fr = pool_free(scratch, s);
     return st ? st : fr;
 }
 
