@@ -1,9 +1,8 @@
 // The extern "C" entry points of include/bssn_b200.h: argument checks and
 // kernel launches.  No entry point allocates device memory except the mesh
 // handle's creation and its first use of a tile shape (task list upload, split
-// scratch) or of the constraints, plan creation, the first diagnostics call of
-// a plan, and single-block right-hand sides (from the library's own
-// stream-ordered pool).
+// scratch), plan creation, the first diagnostics call of a plan, and, from
+// stream-ordered pools, single-block right-hand sides and constraints.
 #include <cuda_runtime.h>
 
 #include <cstring>

@@ -10,8 +10,8 @@
 // The algebra at one node is one function over where the node's derivatives
 // come from.  Single-level meshes run the split right-hand side's derivative
 // pass (rhs_columns.cuh) on the seventeen variables the constraints
-// differentiate, chunk by chunk into the mesh's scratch, and read them back
-// per zone.  Level meshes, and calls that cannot have the scratch, read the
+// differentiate, chunk by chunk into scratch, and read them back per zone.
+// Level meshes, and calls that cannot have scratch, read the
 // stencils straight from the padded block in global memory (cached) with the
 // bit-exact stencils of stencil_exact.cuh; mixed derivatives are then first
 // derivatives of on-the-fly first derivatives, in the reference's order
@@ -27,6 +27,7 @@
 #include "constraints.h"
 #include "kernels.cuh"
 #include "mesh.h"
+#include "pool.h"
 #include "rhs_columns.cuh"
 #include "stencil_exact.cuh"
 
@@ -540,55 +541,59 @@ static ColVars constraint_vars() {
 }
 
 // Single-level meshes: the derivative pass and the algebra, chunk by chunk.
-// Returns BSSN_ENOMEM before any launch when the scratch cannot be had (no
-// device memory, or a capture running and none allocated yet).
-static int constraints_split(MeshState* m, const ConstVars& p, const MutVars& o, cudaStream_t s, bool psi4) {
+// The mesh's scratch belongs to whatever stream its steps run on and is
+// replaced when it grows, so a call on its own takes scratch from a pool of the
+// mesh (kept until the mesh goes): kConsZones zones at most, or what the
+// library's pool keeps when there is no room.  9.0 M nodes in mixed blocks: 8.8
+// ms a million zones at a time, 9.7 with half of that, 13.7 with the 126 k zones
+// of the library's pool.  BSSN_ENOMEM before any launch when there is none (a
+// stream capture, or no memory).
+static int constraints_split(const MeshState* m, const ConstVars& p, const MutVars& o, cudaStream_t s, bool psi4,
+                             double* scratch, int64_t zones) {
     const int64_t nn = (int64_t)m->G[0] * m->G[1] * m->G[2];
     if (nn >= (int64_t(1) << 31)) return BSSN_ENOMEM;  // node indices of the grid arguments are 32-bit
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {  // the legacy stream while another one captures
-        cudaGetLastError();
-        return BSSN_ENOMEM;
+    constexpr int64_t kZoneBytes = kSplitZoneBytes;
+    double* own = nullptr;
+    if (!scratch) {
+        zones = 0;
+        for (size_t k = 0; k < m->sides.size(); k++)
+            zones = std::max(zones, (int64_t)m->default_tasks[k].second *
+                                        tile_zones(default_split_tile(m->sides[k]), m->sides[k]));
+        zones = std::min(zones, kConsZones);
+        if (m->cons_pool.alloc((void**)&own, kZoneBytes * zones, s)) {
+            zones = std::min(zones, (int64_t)kPoolKeepBytes / kZoneBytes);
+            const int st = pool_alloc((void**)&own, kZoneBytes * zones, s);
+            if (st) return st;
+        }
+        scratch = own;
     }
-    // a chunk of a million zones (1.4 GB) is enough when no plan has made the
-    // scratch larger
-    int64_t need = 0;
-    bool known = true;
-    for (int side : m->sides) {
-        const int t = default_split_tile(side);
-        known = known && m->tasks.count(std::make_pair(t, side));
-        if (cap == cudaStreamCaptureStatusNone || known) need = std::max(need, split_need(m, t, side));
-    }
-    need = std::min<int64_t>(need, int64_t(1) << 20);
-    if (cap != cudaStreamCaptureStatusNone && (!known || m->scratch_zones < need)) return BSSN_ENOMEM;
-    int st = mesh_scratch(m, need);
-    if (st) return BSSN_ENOMEM;
     const ZipGrid g{m->G[0], m->G[1], m->G[2]};
     const ColVars vars = constraint_vars();
-    for (int side : m->sides) {
-        const int t = default_split_tile(side);
-        const BrickTask* tk;
-        int nt;
-        st = mesh_tasks_side(m, t, side, &tk, &nt);
-        if (st) return st;
-        st = split_chunks(t, side, p, m->d_axis, m->d_blocks, tk, nt, m->d_scratch, m->scratch_zones, s, g, vars,
+    int st = 0;
+    for (size_t k = 0; k < m->sides.size() && !st; k++) {
+        const int side = m->sides[k], t = default_split_tile(side);
+        st = split_chunks(t, side, p, m->d_axis, m->d_blocks, m->default_tasks[k].first, m->default_tasks[k].second,
+                          scratch, zones, s, g, vars,
                           [&](const BrickTask* tasks, int n, int64_t zs, const int b[2], int nz) {
                               const int parts = (nz + 127) / 128;
                               if (psi4)
                                   constraints_scratch_kernel<true><<<n * parts, 128, 0, s>>>(
-                                      p, o, m->d_blocks, tasks, m->d_scratch, zs, g, b[0], b[1], nz);
+                                      p, o, m->d_blocks, tasks, scratch, zs, g, b[0], b[1], nz);
                               else
                                   constraints_scratch_kernel<false><<<n * parts, 128, 0, s>>>(
-                                      p, o, m->d_blocks, tasks, m->d_scratch, zs, g, b[0], b[1], nz);
+                                      p, o, m->d_blocks, tasks, scratch, zs, g, b[0], b[1], nz);
                               return cuda_status(cudaGetLastError());
                           });
-        if (st) return st;
     }
-    return 0;
+    if (own) {
+        const int fr = pool_free(own, s);
+        if (!st) st = fr;
+    }
+    return st;
 }
 
-int launch_constraints(MeshState* m, const double* const* P, double* const* out,
-                       cudaStream_t s, bool psi4) {
+int launch_constraints(const MeshState* m, const double* const* P, double* const* out,
+                       cudaStream_t s, bool psi4, double* scratch, int64_t zones) {
     ConstVars p;
     MutVars o = {};
     for (int v = 0; v < NVARS; v++) p.p[v] = P[v];
@@ -604,7 +609,7 @@ int launch_constraints(MeshState* m, const double* const* P, double* const* out,
             constraints_levels_kernel<false><<<grid, 256, 0, s>>>(p, o, m->d_blocks, nb, m->lv->zip_src, nn);
         return cuda_status(cudaGetLastError());
     }
-    const int st = constraints_split(m, p, o, s, psi4);
+    const int st = constraints_split(m, p, o, s, psi4, scratch, zones);
     if (st != BSSN_ENOMEM) return st;
     if (m->n_int_chunks == 0) return 0;
     if (psi4)

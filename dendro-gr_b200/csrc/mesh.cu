@@ -140,6 +140,12 @@ int mesh_create(const BssnBlockDesc* blocks, int nblocks, const int32_t G[3],
     if (!st) st = upload(axis, &m->d_axis);
     if (!st) st = upload(pad, &m->d_pad_chunks);
     if (!st) st = upload(inner, &m->d_int_chunks);
+    for (int side : m->sides) {
+        const BrickTask* tk = nullptr;
+        int nt = 0;
+        if (!st) st = mesh_tasks_side(m, default_split_tile(side), side, &tk, &nt);
+        m->default_tasks.push_back({tk, nt});
+    }
     if (st) {
         mesh_destroy(m);
         return st;

@@ -9,12 +9,15 @@
 
 #include "bssn_b200.h"
 #include "levels.h"
+#include "pool.h"
 #include "remesh.h"
 #include "rhs_fused.cuh"
 
 namespace bssn {
 
 constexpr int kAllSides = -1;
+constexpr int64_t kSplitZoneBytes = sizeof(double) * kSplitSlots;
+constexpr int64_t kConsZones = int64_t(1) << 20;  // zones of scratch of one constraints call
 
 // A run of consecutive points of one block handled by one CTA.
 struct Chunk {
@@ -37,6 +40,9 @@ struct MeshState {
     // brick task lists per (tile shape, block side; side 0 = all blocks):
     // (device pointer, count)
     std::map<std::pair<int, int>, std::pair<BrickTask*, int>> tasks;
+    // the lists of the sides' default split tiles, in the order of `sides`; made with the mesh and never changed, for calls that may
+    // run on several threads at once or under a capture
+    std::vector<std::pair<const BrickTask*, int>> default_tasks;
     // partial sums of the constraint-norm reduction (allocated on first use)
     double* d_partial = nullptr;
     // elements (octants) of all blocks and the first element of each block
@@ -61,6 +67,8 @@ struct MeshState {
     // scratch of the split right-hand side (kSplitSlots doubles per zone)
     double* d_scratch = nullptr;
     int64_t scratch_zones = 0;
+    // scratch of constraints called on their own, each call a buffer
+    mutable ScratchPool cons_pool{size_t(kConsZones * kSplitZoneBytes)};
     // multi-level meshes: the level maps (nullptr for single-level meshes,
     // whose zipped state is one node grid of dims G)
     LevelsDev* lv = nullptr;

@@ -379,8 +379,13 @@ static int diag_prepare(Plan* p) {
     return 0;
 }
 
-static int enqueue_diag(Plan* p, double* const* u, const DiagArgs& d, cudaStream_t s) {
+// behind_step: enqueued right behind a step of the plan, whose order on the
+// stream then already owns the mesh's scratch (where the step uses it: a split
+// tile on some side); on their own the diagnostics must not touch it.
+static int enqueue_diag(Plan* p, double* const* u, const DiagArgs& d, cudaStream_t s, bool behind_step) {
     MeshState* m = p->mesh;
+    bool owns = false;
+    for (int side : p->sides) owns = owns || (behind_step && tile_mode(plan_tile(p, side)) == 1);
     double* Pp[NVARS];
     set_ptrs(p->P, m->unzip_size, Pp);
     int st = unzip_all(m, Pp, (const double* const*)u, s);
@@ -388,7 +393,8 @@ static int enqueue_diag(Plan* p, double* const* u, const DiagArgs& d, cudaStream
     const bool psi4 = (p->flags & BSSN_PLAN_DIAG_PSI4) != 0;
     double* cons[6];
     for (int c = 0; c < (psi4 ? 6 : 4); c++) cons[c] = p->cons + (size_t)c * p->n_nodes;
-    st = launch_constraints(m, (const double* const*)Pp, cons, s, psi4);
+    st = launch_constraints(m, (const double* const*)Pp, cons, s, psi4, owns ? m->d_scratch : nullptr,
+                            m->scratch_zones);
     if (st) return st;
     return launch_l2_norms(m, (const double* const*)cons, 4, d.xmin, d.h, d.bh, d.radii, m->d_partial,
                            kNormPartials, d.norms, s);
@@ -396,7 +402,7 @@ static int enqueue_diag(Plan* p, double* const* u, const DiagArgs& d, cudaStream
 
 int plan_diag(Plan* p, double* const* u, const DiagArgs& d, cudaStream_t s) {
     const int st = diag_prepare(p);
-    return st ? st : enqueue_diag(p, u, d, s);
+    return st ? st : enqueue_diag(p, u, d, s, false);
 }
 
 // One RK4 step followed by the diagnostics of the new state, captured as one
@@ -408,7 +414,7 @@ int plan_step_diag(Plan* p, double* const* u, double dt, const DiagArgs& d, cuda
     if (st) return st;
     auto body = [&](cudaStream_t cs) {
         int r = plan_enqueue(p, u, dt, cs);
-        return r ? r : enqueue_diag(p, u, d, cs);
+        return r ? r : enqueue_diag(p, u, d, cs, true);
     };
     if (!(p->flags & BSSN_PLAN_GRAPH)) return body(s);
     double key[14] = {dt, d.xmin[0], d.xmin[1], d.xmin[2], d.h, d.bh[0], d.bh[1], d.bh[2],

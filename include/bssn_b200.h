@@ -179,10 +179,13 @@ int bssn_initial_data_f64(double* const* u_dev, const int32_t G[3],
  * multi-level mesh every zipped node (the level grids back to back) takes
  * the value at the zone that owns it; nodes filled from another level
  * (patch-boundary nodes, coarse nodes under a finer patch) are set to 0, so
- * each physical point carries its value once.  Single-level meshes use the
- * handle's derivative scratch (allocated here, up to 1.4 GB, when neither a
- * plan nor bssn_rhs_blocks_f64 has; without it -- no memory, or a stream
- * capture before it exists -- a slower kernel that needs none runs). */
+ * each physical point carries its value once.  On single-level meshes the
+ * derivatives pass through scratch of the call's own, from a stream-ordered pool
+ * that the handle keeps (at most 1.4 GB; the right-hand side's scratch is not
+ * used, so calls may run beside steps of the mesh); under a stream capture,
+ * without memory, and on multi-level meshes a slower kernel runs that needs
+ * none.  The two round the outer stage of the mixed derivatives differently
+ * (1e-12 of the largest value). */
 int bssn_constraints_f64(bssn_mesh mesh, const double* const* unzip_dev,
                          double* const* cons_dev, bssn_stream_t stream);
 /* The same constraints plus the Weyl scalar psi4 for gravitational-wave

@@ -143,3 +143,75 @@ def test_constraints_with_and_without_scratch():
         torch.cuda.synchronize()
         out.append(cons.cpu().numpy())
     assert ol.rel_err(out[0], out[1]).max() <= 1e-12
+
+
+def _constraints(B, mesh, P, psi4, stream=None):
+    n = mesh.spec.n_nodes
+    out = torch.zeros((6 if psi4 else 4, n), dtype=torch.float64, device="cuda")
+    fn = B.lib.bssn_constraints_psi4_f64 if psi4 else B.lib.bssn_constraints_f64
+    fn.argtypes = [C.c_void_p] * 4
+    ptrs = (C.c_void_p * out.shape[0])(*[out.data_ptr() + 8 * n * c for c in range(out.shape[0])])
+    B.check(fn(mesh.h, B.ptrs(P), ptrs, B.stream_ptr(stream)), "constraints")
+    return out
+
+
+@pytest.mark.parametrize("psi4", [False, True])
+def test_captured_constraints_outlive_scratch_growth(psi4):
+    """Constraints captured on a mesh that already has derivative scratch,
+    replayed after a plan and a right-hand side have replaced that scratch: the
+    graph holds nothing of the mesh that can be freed.  The mesh needs several
+    scratch-fuls of the pool's size on every side but 13.  The forms with and
+    without scratch round the outer stage of the mixed derivatives differently:
+    1e-12 of the largest value."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(1, (2, 2, 2), seed=20261203, xmin=-8.25)
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    mesh = B.Mesh(spec)
+    P = torch.zeros((24, mesh.n_unzip), dtype=torch.float64, device="cuda")
+    mesh.unzip(P, U)
+    R = torch.zeros_like(P)
+    mesh.rhs(R, P, B.default_params(), tile=6)  # scratch for 7x7 columns
+    eager = _constraints(B, mesh, P, psi4)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        captured = _constraints(B, mesh, P, psi4)
+    plan = B.RK4Plan(mesh, B.default_params(), B.PLAN_GRAPH)
+    mesh.rhs(R, P, B.default_params())
+    captured.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert ol.rel_err(eager.cpu().numpy(), captured.cpu().numpy()).max() <= 1e-12
+    plan.close()
+
+
+def test_constraints_beside_right_hand_sides():
+    """Constraints on one stream while right-hand sides and steps of the same
+    mesh run on another: each has its own scratch, so both give what they give
+    alone."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(1, (2, 1, 1), seed=5, xmin=-8.25)
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    prm = B.default_params()
+    mesh = B.Mesh(spec)
+    P = torch.zeros((24, mesh.n_unzip), dtype=torch.float64, device="cuda")
+    mesh.unzip(P, U)
+    want_r = torch.zeros_like(P)
+    mesh.rhs(want_r, P, prm)
+    want_c = _constraints(B, mesh, P, True)
+    torch.cuda.synchronize()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    rhs, cons = [], []
+    for _ in range(4):
+        rhs.append(torch.zeros_like(P))
+        cons.append(torch.zeros_like(want_c))
+    torch.cuda.synchronize()
+    for k in range(4):
+        mesh.rhs(rhs[k], P, prm, stream=a)
+        with torch.cuda.stream(b):
+            cons[k] = _constraints(B, mesh, P, True, stream=b)
+    torch.cuda.synchronize()
+    for k in range(4):
+        assert torch.equal(rhs[k], want_r) and torch.equal(cons[k], want_c)
