@@ -136,9 +136,10 @@ int bssn_rhs_blocks_f64(bssn_mesh mesh, double* const* rhs_dev, const double* co
         lists.push_back(l);
     }
     int r = bssn::mesh_scratch(m, need);
+    double* scratch = m->scratch.on(S(stream));
     for (size_t k = 0; k < lists.size() && !r; k++)
         r = bssn::launch_rhs_tasks(lists[k].tile, lists[k].side, A, m->d_blocks, lists[k].tasks, lists[k].ntasks, S(stream),
-                                   m->d_scratch, m->scratch_zones);
+                                   scratch, m->scratch_zones());
     return r;
 }
 

@@ -169,7 +169,6 @@ void mesh_destroy(MeshState* m) {
     cudaFree(m->d_fchunk_first);
     cudaFree(m->d_fpart);
     for (auto& t : m->tasks) cudaFree(t.second.first);
-    cudaFree(m->d_scratch);
     if (m->lv) {
         levels_free(m->lv);
         delete m->lv;
@@ -178,17 +177,7 @@ void mesh_destroy(MeshState* m) {
 }
 
 int mesh_scratch(MeshState* m, int64_t zones) {
-    if (zones > kSplitScratchZonesMax) zones = kSplitScratchZonesMax;
-    if (zones <= m->scratch_zones) return 0;
-    cudaFree(m->d_scratch);
-    m->d_scratch = nullptr;
-    m->scratch_zones = 0;
-    if (cudaMalloc((void**)&m->d_scratch, sizeof(double) * kSplitSlots * zones) != cudaSuccess) {
-        cudaGetLastError();
-        return BSSN_ENOMEM;
-    }
-    m->scratch_zones = zones;
-    return 0;
+    return m->scratch.grow((size_t)(std::min(zones, kSplitScratchZonesMax) * kSplitZoneBytes));
 }
 
 int64_t split_need(MeshState* m, int tile, int side) {

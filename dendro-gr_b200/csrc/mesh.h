@@ -65,8 +65,8 @@ struct MeshState {
     // every side under the key kAllSides
     std::map<int, int> tuned;
     // scratch of the split right-hand side (kSplitSlots doubles per zone)
-    double* d_scratch = nullptr;
-    int64_t scratch_zones = 0;
+    GrowingScratch scratch;
+    int64_t scratch_zones() const { return (int64_t)scratch.bytes() / kSplitZoneBytes; }
     // scratch of constraints called on their own, each call a buffer
     mutable ScratchPool cons_pool{size_t(kConsZones * kSplitZoneBytes)};
     // multi-level meshes: the level maps (nullptr for single-level meshes,

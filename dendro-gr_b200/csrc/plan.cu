@@ -177,6 +177,7 @@ bool plan_zipped_rhs(const Plan* p) {
 // write R, or Rz when plan_zipped_rhs.
 int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src) {
     MeshState* m = p->mesh;
+    double* scratch = m->scratch.on(s);
     RhsArgs A;
     A.prm = p->prm;
     A.axis = m->d_axis;
@@ -195,7 +196,7 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
             int nt;
             st = mesh_tasks_side(m, t, side, &tk, &nt);
             if (!st)
-                st = launch_rhs_tasks(t, side, A, m->d_blocks, tk, nt, s, m->d_scratch, m->scratch_zones, tm,
+                st = launch_rhs_tasks(t, side, A, m->d_blocks, tk, nt, s, scratch, m->scratch_zones(), tm,
                                       m->G);
             if (st) break;
         }
@@ -230,8 +231,8 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
                 const int per = bricks_per_block(t, b.sz);
                 if (!st && (j + 1) * per > nt) st = BSSN_ESTATE;
                 if (!st)
-                    st = launch_rhs_tasks(t, b.sz, A, m->d_blocks, tk + (size_t)j * per, per, s, m->d_scratch,
-                                          m->scratch_zones, tm);
+                    st = launch_rhs_tasks(t, b.sz, A, m->d_blocks, tk + (size_t)j * per, per, s, scratch,
+                                          m->scratch_zones(), tm);
             } else {
                 st = launch_rhs_single(t, A, b, s);
             }
@@ -254,8 +255,8 @@ int plan_rhs(Plan* p, cudaStream_t s, KernelTimer* tm, const double* const* src)
         int nt;
         int st = mesh_tasks_side(m, t, side, &tk, &nt);
         if (!st)
-            st = launch_rhs_tasks(t, side, A, m->d_blocks, tk, nt, s, m->d_scratch,
-                                  m->scratch_zones, tm, zrhs ? m->G : nullptr, direct);
+            st = launch_rhs_tasks(t, side, A, m->d_blocks, tk, nt, s, scratch,
+                                  m->scratch_zones(), tm, zrhs ? m->G : nullptr, direct);
         if (st) return st;
     }
     return 0;
@@ -393,8 +394,8 @@ static int enqueue_diag(Plan* p, double* const* u, const DiagArgs& d, cudaStream
     const bool psi4 = (p->flags & BSSN_PLAN_DIAG_PSI4) != 0;
     double* cons[6];
     for (int c = 0; c < (psi4 ? 6 : 4); c++) cons[c] = p->cons + (size_t)c * p->n_nodes;
-    st = launch_constraints(m, (const double* const*)Pp, cons, s, psi4, owns ? m->d_scratch : nullptr,
-                            m->scratch_zones);
+    st = launch_constraints(m, (const double* const*)Pp, cons, s, psi4, owns ? m->scratch.on(s) : nullptr,
+                            m->scratch_zones());
     if (st) return st;
     return launch_l2_norms(m, (const double* const*)cons, 4, d.xmin, d.h, d.bh, d.radii, m->d_partial,
                            kNormPartials, d.norms, s);
@@ -437,6 +438,7 @@ int plan_step_diag(Plan* p, double* const* u, double dt, const DiagArgs& d, cuda
 // and keep the fastest.  Blocking.
 int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* times_out) {
     MeshState* m = p->mesh;
+    double* scratch = m->scratch.on(s);
     RhsArgs A;
     A.prm = p->prm;
     A.axis = m->d_axis;
@@ -474,7 +476,7 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
         ms = 1e30f;
         for (int k = 0; k <= reps && !r; k++) {
             cudaEventRecord(e0, s);
-            r = launch_rhs_tasks(t, side, A, m->d_blocks, tk, ntask, s, m->d_scratch, m->scratch_zones, nullptr, zg);
+            r = launch_rhs_tasks(t, side, A, m->d_blocks, tk, ntask, s, scratch, m->scratch_zones(), nullptr, zg);
             cudaEventRecord(e1, s);
             if (r) break;
             cudaEventSynchronize(e1);
@@ -609,7 +611,7 @@ int plan_launches_per_step(Plan* p) {
             const BrickTask* tk;
             int nt = 0;
             if (mesh_tasks_side(m, t, side, &tk, &nt)) return -1;
-            rhs += rhs_launch_count(t, nt, m->scratch_zones, side);
+            rhs += rhs_launch_count(t, nt, m->scratch_zones(), side);
         }
     }
     if (m->lv) {  // interpolation passes, ghost fill, stage, one launch per non-empty sync segment

@@ -55,6 +55,53 @@ ScratchPool::~ScratchPool() {
     if (pool_) cudaMemPoolDestroy(pool_);
 }
 
+int GrowingScratch::grow(size_t bytes) {
+    if (bytes <= bytes_) return 0;
+    auto make = [](size_t n) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, n) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return static_cast<double*>(p);
+    };
+    double* p = make(bytes);
+    if (p) {
+        if (captured_)
+            kept_.push_back(p_);
+        else
+            cudaFree(p_);
+    } else {
+        if (captured_ || !p_) return BSSN_ENOMEM;
+        // both do not fit at once: the old one goes first
+        cudaFree(p_);
+        p = make(bytes);
+        if (!p) {
+            p_ = make(bytes_);
+            if (!p_) bytes_ = 0;
+            return BSSN_ENOMEM;
+        }
+    }
+    p_ = p;
+    bytes_ = bytes;
+    captured_ = false;
+    return 0;
+}
+
+double* GrowingScratch::on(cudaStream_t s) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess)
+        cudaGetLastError();  // the legacy stream while another one captures: the launch reports it
+    else if (cap != cudaStreamCaptureStatusNone)
+        captured_ = true;
+    return p_;
+}
+
+GrowingScratch::~GrowingScratch() {
+    if (p_) cudaFree(p_);
+    for (double* p : kept_) cudaFree(p);
+}
+
 int pool_alloc(void** p, size_t bytes, cudaStream_t s) {
     // never destroyed: calls may come from any thread until the process ends
     static std::mutex& mu = *new std::mutex;

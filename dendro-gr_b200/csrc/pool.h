@@ -5,6 +5,7 @@
 #include <stddef.h>
 
 #include <mutex>
+#include <vector>
 
 namespace bssn {
 
@@ -26,6 +27,29 @@ private:
     std::mutex mu_;
     cudaMemPool_t pool_ = nullptr;
     size_t keep_;
+};
+
+// One buffer that grows.  A buffer that a captured launch may have recorded is
+// kept when a larger one takes its place, until the object goes, so that the
+// graph stays valid; any other is freed.  A growth that fails leaves a buffer of
+// the old size.
+class GrowingScratch {
+public:
+    GrowingScratch() = default;
+    ~GrowingScratch();
+    GrowingScratch(const GrowingScratch&) = delete;
+    GrowingScratch& operator=(const GrowingScratch&) = delete;
+    // Makes the buffer hold at least `bytes` (outside stream captures).
+    int grow(size_t bytes);
+    size_t bytes() const { return bytes_; }
+    // The buffer, for launches on s.
+    double* on(cudaStream_t s);
+
+private:
+    double* p_ = nullptr;
+    size_t bytes_ = 0;
+    bool captured_ = false;
+    std::vector<double*> kept_;
 };
 
 // Bytes the library's own pool of each device keeps (the split scratch of the

@@ -215,3 +215,34 @@ def test_constraints_beside_right_hand_sides():
     torch.cuda.synchronize()
     for k in range(4):
         assert torch.equal(rhs[k], want_r) and torch.equal(cons[k], want_c)
+
+
+def test_captured_right_hand_side_outlives_scratch_growth():
+    """A right-hand side captured with the scratch of narrow columns, replayed
+    after wider ones and a plan have replaced that scratch, and that plan's own
+    graph after another growth."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(0, (4, 4, 4), seed=0, xmin=-8.25)
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    prm = B.default_params()
+    mesh = B.Mesh(spec)
+    P = torch.zeros((24, mesh.n_unzip), dtype=torch.float64, device="cuda")
+    mesh.unzip(P, U)
+    want, got = torch.zeros_like(P), torch.zeros_like(P)
+    mesh.rhs(want, P, prm, tile=6)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        mesh.rhs(got, P, prm, tile=6)
+    for t in range(len(B.tiles())):
+        if B.tile_mode(t) == 1:
+            mesh.rhs(torch.zeros_like(P), P, prm, tile=t)
+    plan = B.RK4Plan(mesh, prm, B.PLAN_GRAPH)
+    V = U.clone()
+    plan.step(V, 1e-3)
+    got.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    plan.close()

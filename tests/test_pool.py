@@ -8,7 +8,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 
-def test_pool_creation_is_tried_again(tmp_path):
+def test_scratch_over_a_fake_runtime(tmp_path):
     if not os.path.isfile(os.path.join(CUDA, "include", "cuda_runtime.h")):
         pytest.skip("no CUDA headers")
     exe = str(tmp_path / "pool")
