@@ -433,25 +433,34 @@ int plan_step_diag(Plan* p, double* const* u, double dt, const DiagArgs& d, cuda
 }
 
 // Project-written autotuner: for every block-size bucket of the mesh, time
-// the fused right-hand side of that bucket with every compiled tile shape on
-// the current padded state (CUDA events, best of `reps` after one warm-up)
+// the right-hand side of that bucket with every compiled tile shape, in the
+// form the plan's steps run it (CUDA events, best of `reps` after one warm-up),
 // and keep the fastest.  Blocking.
+//
+// Plans that can run the zipped form time it: the state u read and the
+// right-hand side written on the node grid, owned zones only (a 13^3 block has
+// 216 of 343).  A tile without that form is timed on the padded state for the
+// caller's table but not chosen: with it on one side the whole mesh would step
+// through ghost fill, padded right-hand sides and gather again, which its own
+// time does not hold.
 int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* times_out) {
     MeshState* m = p->mesh;
     double* scratch = m->scratch.on(s);
-    RhsArgs A;
-    A.prm = p->prm;
-    A.axis = m->d_axis;
+    RhsArgs A, Z;  // padded and zipped form
+    A.prm = Z.prm = p->prm;
+    A.axis = Z.axis = m->d_axis;
     A.drop = m->lv ? m->lv->drop : nullptr;
+    const bool zipped = p->Rz && !(p->flags & BSSN_PLAN_PER_BLOCK) && !m->lv;
     int st = 0;
-    if (p->direct) {  // split tiles on the zipped state u
+    if (zipped) {
         double* Rz[NVARS];
         set_ptrs(p->Rz, p->n_nodes, Rz);
         for (int v = 0; v < NVARS; v++) {
-            A.u.p[v] = u[v];
-            A.rhs.p[v] = Rz[v];
+            Z.u.p[v] = u[v];
+            Z.rhs.p[v] = Rz[v];
         }
-    } else {
+    }
+    if (!p->direct) {
         double* Pp[NVARS];
         set_ptrs(p->P, m->unzip_size, Pp);
         st = unzip_all(m, Pp, (const double* const*)u, s);
@@ -463,7 +472,7 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
             A.rhs.p[v] = Rp[v];
         }
     }
-    const int32_t* zg = p->direct ? m->G : nullptr;
+    auto zip_form = [&](int t) { return zipped && tile_zipped(tile_mode(t)); };
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -476,7 +485,8 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
         ms = 1e30f;
         for (int k = 0; k <= reps && !r; k++) {
             cudaEventRecord(e0, s);
-            r = launch_rhs_tasks(t, side, A, m->d_blocks, tk, ntask, s, scratch, m->scratch_zones(), nullptr, zg);
+            r = launch_rhs_tasks(t, side, zip_form(t) ? Z : A, m->d_blocks, tk, ntask, s, scratch, m->scratch_zones(),
+                                 nullptr, zip_form(t) ? m->G : nullptr);
             cudaEventRecord(e1, s);
             if (r) break;
             cudaEventSynchronize(e1);
@@ -527,7 +537,7 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
             if (plan_runs_tile(p, t, side)) st = time_tile(t, side, tbest);
             if (st) break;
             if (times_out) times_out[idx * nt + t] = tbest;
-            if (tbest < best) {
+            if (tbest < best && (!zipped || zip_form(t))) {
                 best = tbest;
                 best_t = t;
             }

@@ -449,7 +449,9 @@ int bssn_rk4_plan_copy_diag_fields(bssn_rk4_plan plan, double* const* dst_dev, i
                                    bssn_stream_t stream);
 /* Autotuner: times every tile the plan can run (direct plans: split tiles
  * only) on every block-size bucket of the mesh with the state u_dev (best of
- * reps) and keeps the fastest per bucket in the mesh handle.  Blocking.
+ * reps), in the form its steps run it, and keeps the fastest per bucket in the
+ * mesh handle.  On single-level meshes fused tiles are timed on padded blocks
+ * and not chosen: one would take the whole mesh back to them.  Blocking.
  * times (optional): nbuckets x bssn_tile_count() milliseconds, buckets in
  * increasing side order, 1e30 for tiles not timed. */
 int bssn_rk4_plan_autotune(bssn_rk4_plan plan, double* const* u_dev, int reps,

@@ -246,3 +246,26 @@ def test_captured_right_hand_side_outlives_scratch_growth():
     torch.cuda.synchronize()
     assert torch.equal(got, want)
     plan.close()
+
+
+def _kernels(f):
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        f()
+        torch.cuda.synchronize()
+    return {e.name for e in p.events() if "bssn" in e.name}
+
+
+@pytest.mark.parametrize("flags", [0, 4, 8])  # default, block by block, direct
+def test_autotune_times_the_kernels_the_step_runs(flags):
+    """Every derivative and equation kernel of a step under the chosen tiles is
+    one that the tuner launched to choose them."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(1, (2, 1, 1), seed=20261203, xmin=-8.25)
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    plan = B.RK4Plan(B.Mesh(spec), B.default_params(), flags)
+    tuned = _kernels(lambda: plan.autotune(U, reps=1))
+    step = {k for k in _kernels(lambda: plan.step(U, 1e-3)) if "column_kernel" in k or "eq_kernel" in k}
+    plan.close()
+    assert step and step <= tuned, step - tuned
