@@ -248,6 +248,41 @@ def test_captured_right_hand_side_outlives_scratch_growth():
     plan.close()
 
 
+@pytest.mark.parametrize("faces", [True, False])
+def test_zipped_steps_under_every_split_tile(faces):
+    """A step through the zipped form (node offsets, zero outside the grid,
+    owned zones only) under every split tile, on every side that takes it:
+    the same bits as the padded block loop, with the domain's physical faces
+    and with none (every block interior, zeros beyond the grid)."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(1, (2, 2, 2), seed=20261203, xmin=-8.25)
+    assert set(spec.sides.tolist()) == {13, 19, 31, 55}
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    if not faces:
+        for b in range(spec.nblocks):
+            spec.blocks[b].bflag = 0
+    mesh = B.Mesh(spec)
+    prm = B.default_params()
+    ref = U.clone()
+    plan = B.RK4Plan(mesh, prm, B.PLAN_PER_BLOCK)
+    plan.step(ref, 1e-6)
+    torch.cuda.synchronize()
+    plan.close()
+    assert bool(torch.isfinite(ref).all()) and not torch.equal(ref, U)
+    for flags in (0, B.PLAN_DIRECT):
+        plan = B.RK4Plan(mesh, prm, flags)
+        for t in range(len(B.tiles())):
+            if B.tile_mode(t) != 1:
+                continue
+            plan.set_tile(t)
+            V = U.clone()
+            plan.step(V, 1e-6)
+            torch.cuda.synchronize()
+            assert torch.equal(V, ref), (flags, t)
+        plan.close()
+
+
 def _kernels(f):
     from torch.profiler import ProfilerActivity, profile
     with profile(activities=[ProfilerActivity.CUDA]) as p:
