@@ -30,8 +30,9 @@
 // cooperative halo pass, closures by per-term constant tables) issued about
 // 430 instructions with 52 shared loads.  Derivative passes of one RK4 step:
 // 19.8 M zones in 4,108 mixed blocks 58.2 -> 39 ms, a 2,708-block level mesh
-// 9.3 -> 7.2 ms, 512 blocks of 13^3 (176 k zones, 58 % of the blocks on the
-// boundary) 1.09 -> 0.82 ms.
+// 9.3 -> 7.2 ms.  On 13^3 blocks, where a thread marches thirteen planes for
+// seven, it gained on boundary blocks only and lost 16-31 % of the padded pass
+// elsewhere; they run a form of their own (rhs_cube.cuh).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -120,12 +121,25 @@ __constant__ double kZCloD1[2][3][5] = {
     {{-25, 48, -36, 16, -3}, {-3, -10, 18, -6, 1}, {1, -8, 0, 8, -1}},
     {{1, -8, 0, 8, -1}, {-1, 6, -18, 10, 3}, {3, -16, 36, -48, 25}}};
 
-__device__ __forceinline__ void z_closures(bool lo, const double (&u)[6], const AxisCoef& cf, double d1[3],
-                                           double d2[3], double ko[3]) {
+// One-sided closures along a line that ends at a physical face, from its six
+// points next to the face.
+__device__ __forceinline__ void z_closures_d1(bool lo, const double (&u)[6], const AxisCoef& cf, double d1[3]) {
     if (lo) {
         { const double c[5] = {-25, 48, -36, 16, -3}; const int p[5] = {0, 1, 2, 3, 4}; d1[0] = fold6(c, u, p); }
         { const double c[5] = {-3, -10, 18, -6, 1}; const int p[5] = {0, 1, 2, 3, 4}; d1[1] = fold6(c, u, p); }
         { const double c[4] = {1, -8, 8, -1}; const int p[4] = {0, 1, 3, 4}; d1[2] = fold6(c, u, p); }
+    } else {
+        { const double c[4] = {1, -8, 8, -1}; const int p[4] = {1, 2, 4, 5}; d1[0] = fold6(c, u, p); }
+        { const double c[5] = {-1, 6, -18, 10, 3}; const int p[5] = {1, 2, 3, 4, 5}; d1[1] = fold6(c, u, p); }
+        { const double c[5] = {3, -16, 36, -48, 25}; const int p[5] = {1, 2, 3, 4, 5}; d1[2] = fold6(c, u, p); }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++) d1[q] = __dmul_rn(d1[q], cf.ih12);
+}
+__device__ __forceinline__ void z_closures(bool lo, const double (&u)[6], const AxisCoef& cf, double d1[3],
+                                           double d2[3], double ko[3]) {
+    z_closures_d1(lo, u, cf, d1);
+    if (lo) {
         { const double c[6] = {45, -154, 214, -156, 61, -10}; const int p[6] = {0, 1, 2, 3, 4, 5}; d2[0] = fold6(c, u, p); }
         { const double c[6] = {10, -15, -4, 14, -6, 1}; const int p[6] = {0, 1, 2, 3, 4, 5}; d2[1] = fold6(c, u, p); }
         { const double c[5] = {-1, 16, -30, 16, -1}; const int p[5] = {0, 1, 2, 3, 4}; d2[2] = fold6(c, u, p); }
@@ -133,9 +147,6 @@ __device__ __forceinline__ void z_closures(bool lo, const double (&u)[6], const 
         { const double c[5] = {1, -6, 12, -10, 3}; const int p[5] = {4, 3, 2, 1, 0}; ko[1] = fold6(c, u, p); }
         { const double c[6] = {1, -6, 15, -19, 12, -3}; const int p[6] = {5, 4, 3, 2, 1, 0}; ko[2] = fold6(c, u, p); }
     } else {
-        { const double c[4] = {1, -8, 8, -1}; const int p[4] = {1, 2, 4, 5}; d1[0] = fold6(c, u, p); }
-        { const double c[5] = {-1, 6, -18, 10, 3}; const int p[5] = {1, 2, 3, 4, 5}; d1[1] = fold6(c, u, p); }
-        { const double c[5] = {3, -16, 36, -48, 25}; const int p[5] = {1, 2, 3, 4, 5}; d1[2] = fold6(c, u, p); }
         { const double c[5] = {-1, 16, -30, 16, -1}; const int p[5] = {1, 2, 3, 4, 5}; d2[0] = fold6(c, u, p); }
         { const double c[6] = {1, -6, 14, -4, -15, 10}; const int p[6] = {0, 1, 2, 3, 4, 5}; d2[1] = fold6(c, u, p); }
         { const double c[6] = {-10, 61, -156, 214, -154, 45}; const int p[6] = {0, 1, 2, 3, 4, 5}; d2[2] = fold6(c, u, p); }
@@ -146,7 +157,6 @@ __device__ __forceinline__ void z_closures(bool lo, const double (&u)[6], const 
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         const int cs = lo ? q : 3 + q;
-        d1[q] = __dmul_rn(d1[q], cf.ih12);
         d2[q] = __dmul_rn(d2[q], cf.ih2_12);
         ko[q] = __ddiv_rn(ko[q], closure_smr(cs, cf));
     }

@@ -6,7 +6,7 @@
 // registers and one CTA per SM, so it stalls on instruction fetch and on
 // FP64 latency.  Here:
 //   * column_kernel (rhs_columns.cuh) marches columns of each variable along
-//     z and writes every zone's gradient, second derivatives and summed KO
+//     z, or cube_kernel (rhs_cube.cuh) takes whole 13^3 blocks, and writes every zone's gradient, second derivatives and summed KO
 //     term to a scratch array;
 //   * eq_kernel evaluates the equations per zone (rhs_equations.cuh, the same
 //     code as the fused kernel) reading those derivatives back.
@@ -25,6 +25,7 @@
 #include "pool.h"
 #include "rhs_brick.cuh"
 #include "rhs_columns.cuh"
+#include "rhs_cube.cuh"
 #include "rhs_equations.cuh"
 #include "rhs_fused.cuh"
 
@@ -181,6 +182,11 @@ const SplitEntry* split_table(int* count) {
     return table;
 }
 
+// Whole 13^3 blocks run the cube form of the derivative pass, padded or from
+// the node grid, few or many, with faces or without (64 blocks 14 us, 25 as
+// columns; 8,000 blocks 1.57 ms, 1.97).
+bool takes_cube(const SplitEntry& t, int side) { return side == Cube::S && t.bx == Cube::N && t.by == Cube::N; }
+
 }  // namespace
 
 int split_shape_count() {
@@ -224,6 +230,7 @@ long split_selfcheck(int shape) {
     const int B[2] = {t.bx, t.by}, TX = t.bx + 2 * PW, T = t.threads;
     long bad = 0;
     if (t.v2 * t.g2 < kSecondVars || t.v1 * t.g1 < kFirstVars) bad++;
+    if (takes_cube(t, Cube::S)) bad += cube_selfcheck();
     auto case_of = [](int a, int s, int faces) {  // -1: centred
         if (!faces) return -1;
         return a <= 5 ? a - 3 : a >= s - 6 ? a - (s - 9) : -1;
@@ -274,6 +281,11 @@ int prepare_split(int shape) {
     int st = set_smem_limit((const void*)t[shape].deriv, (int)t[shape].smem);
     if (!st) st = set_smem_limit((const void*)t[shape].deriv_one, (int)t[shape].smem);
     if (!st) st = set_smem_limit((const void*)t[shape].deriv_zip, (int)t[shape].smem);
+    if (!st && takes_cube(t[shape], Cube::S)) {
+        st = set_smem_limit((const void*)cube_kernel<false>, (int)Cube::SMEM);
+        if (!st) st = set_smem_limit((const void*)cube_kernel<true>, (int)Cube::SMEM);
+        if (!st) st = set_smem_limit((const void*)cube_one_kernel, (int)Cube::SMEM);
+    }
     if (!st) st = set_smem_limit((const void*)eq_kernel, (int)eq_smem_bytes());
     if (!st) st = set_smem_limit((const void*)eq_one_kernel, (int)eq_smem_bytes());
     return st;
@@ -299,8 +311,12 @@ int split_shape_chunks(int shape, int side, const ConstVars& u, const AxisCoef* 
     for (int64_t c0 = 0; c0 < ntasks; c0 += chunk) {
         const int n = (int)(ntasks - c0 < chunk ? ntasks - c0 : chunk);
         if (tm && (st = tm->start(KernelTimer::DERIV, s))) return st;
-        (zip_in ? t.deriv_zip : t.deriv)<<<n * groups, t.threads, t.smem, s>>>(
-            u, blocks_dev, axis, tasks_dev + c0, scratch, zs, g, nz, vars);
+        if (takes_cube(t, side))
+            (zip_in ? cube_kernel<true> : cube_kernel<false>)<<<n * (vars.n2 + vars.n1), Cube::T, Cube::SMEM, s>>>(
+                u, blocks_dev, axis, tasks_dev + c0, n, scratch, zs, g, cube_vars(vars));
+        else
+            (zip_in ? t.deriv_zip : t.deriv)<<<n * groups, t.threads, t.smem, s>>>(
+                u, blocks_dev, axis, tasks_dev + c0, scratch, zs, g, nz, vars);
         st = cuda_status(cudaGetLastError());
         if (!st && tm) st = tm->stop(s);
         if (!st) st = after(tasks_dev + c0, n, zs, b, nz);
@@ -339,7 +355,11 @@ int launch_rhs_split_single(int shape, const RhsArgs& A, const BssnBlockDesc& bl
     SplitOne one;
     one.blk = blk;
     for (int d = 0; d < 3; d++) one.axis[d] = axis_coef((blk.ptmax[d] - blk.ptmin[d]) / (blk.sz - 1));
-    t.deriv_one<<<bricks * (t.g2 + t.g1), t.threads, t.smem, s>>>(A.u, one, scratch, zs, nz, all_vars());
+    const ColVars all = all_vars();
+    if (takes_cube(t, blk.sz))
+        cube_one_kernel<<<all.n2 + all.n1, Cube::T, Cube::SMEM, s>>>(A.u, one, scratch, zs, cube_vars(all));
+    else
+        t.deriv_one<<<bricks * (t.g2 + t.g1), t.threads, t.smem, s>>>(A.u, one, scratch, zs, nz, all);
     st = cuda_status(cudaGetLastError());
     if (!st) {
         const int parts = (nz + kEqThreads - 1) / kEqThreads;

@@ -145,6 +145,24 @@ def test_constraints_with_and_without_scratch():
     assert ol.rel_err(out[0], out[1]).max() <= 1e-12
 
 
+def test_cube_form_over_more_blocks_than_a_group():
+    """13^3 blocks in a list longer than the cube form's group of blocks, the
+    last group a part of one, on boundary, edge, corner and interior blocks:
+    the same bits as columns."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(0, (11, 11, 11), seed=0, xmin=-8.25)
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-3)
+    mesh = B.Mesh(spec)
+    P = torch.zeros((24, mesh.n_unzip), dtype=torch.float64, device="cuda")
+    mesh.unzip(P, U)
+    cube, cols = torch.zeros_like(P), torch.zeros_like(P)
+    mesh.rhs(cube, P, B.default_params(), tile=6)
+    mesh.rhs(cols, P, B.default_params(), tile=3)
+    torch.cuda.synchronize()
+    assert torch.equal(cube, cols)
+
+
 def _constraints(B, mesh, P, psi4, stream=None):
     n = mesh.spec.n_nodes
     out = torch.zeros((6 if psi4 else 4, n), dtype=torch.float64, device="cuda")
