@@ -203,6 +203,8 @@ uint64_t morton_key(const BssnBlockDesc& b) {
 }  // namespace
 
 int mesh_tasks_side(MeshState* m, int tile, int side, const BrickTask** tasks, int* ntasks) {
+    if (tile < 0 || tile >= tile_count()) return BSSN_EINVAL;
+    tile = tile_canonical(tile);
     const auto key = std::make_pair(tile, side);
     auto it = m->tasks.find(key);
     if (it == m->tasks.end()) {

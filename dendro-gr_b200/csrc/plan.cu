@@ -505,6 +505,10 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
         std::vector<float> tt(nt, 1e30f);
         for (int t = 0; t < nt && !st; t++) {
             if (!tile_zipped(tile_mode(t))) continue;
+            if (tile_canonical(t) != t) {
+                tt[t] = tt[tile_canonical(t)];
+                continue;
+            }
             float sum = 0;
             for (int side : p->sides) {
                 float ms = 0;
@@ -532,9 +536,13 @@ int plan_autotune(Plan* p, double* const* u, int reps, cudaStream_t s, float* ti
     for (int side : p->sides) {
         float best = 1e30f;
         int best_t = 0;
+        std::vector<float> ms(nt, 1e30f);
         for (int t = 0; t < nt; t++) {
-            float tbest = 1e30f;
-            if (plan_runs_tile(p, t, side)) st = time_tile(t, side, tbest);
+            float& tbest = ms[t];
+            if (tile_canonical(t) != t)
+                tbest = ms[tile_canonical(t)];
+            else if (plan_runs_tile(p, t, side))
+                st = time_tile(t, side, tbest);
             if (st) break;
             if (times_out) times_out[idx * nt + t] = tbest;
             if (tbest < best && (!zipped || zip_form(t))) {

@@ -198,8 +198,18 @@ bool tile_fits(int tile, int side) {
     int c;
     const TileEntry* tab = tile_table(&c);
     if (tile < 0 || tile >= c) return false;
-    // bricks of the small shapes clip to any block
-    return tab[tile].mode != 1 || tab[tile].bx <= 13 || tab[tile].bx <= side - 2 * PW;
+    // bricks of the small shapes clip to any block; whole layers of a larger one
+    // (13x13 on 13^3: 12.2 ms against 5.7, and 3.4 times its scratch) do not
+    const TileEntry& t = tab[tile];
+    return t.mode != 1 || t.bx <= side - 2 * PW || t.bx * t.by <= 81;
+}
+
+int tile_canonical(int tile) {
+    int c;
+    const TileEntry* tab = tile_table(&c);
+    for (int t = 0; t < tile; t++)
+        if (tab[t].mode == tab[tile].mode && tab[t].shape == tab[tile].shape && tab[t].mode == 1) return t;
+    return tile;
 }
 
 // Host replay of the brick kernel's shared-memory indexing: for a tile

@@ -63,6 +63,9 @@ int tile_zones(int tile, int side);
 // whether a tile runs on blocks of padded side `side`: not when its brick is
 // wider than their interior
 bool tile_fits(int tile, int side);
+// the first tile of the same kernel: ids that differ in name only share their
+// lists and their time
+int tile_canonical(int tile);
 long tile_selfcheck(int tile);
 int prepare_all_tiles();
 int tile_info(int tile, int info[4]);

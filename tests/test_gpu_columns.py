@@ -322,3 +322,19 @@ def test_autotune_times_the_kernels_the_step_runs(flags):
     step = {k for k in _kernels(lambda: plan.step(U, 1e-3)) if "column_kernel" in k or "eq_kernel" in k}
     plan.close()
     assert step and step <= tuned, step - tuned
+
+
+def test_tiles_that_do_not_suit_a_side():
+    """Whole-layer tiles of larger blocks leave 13^3 blocks to their default;
+    tiles of the same kernel are timed once."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(0, (2, 2, 2), seed=0, xmin=-8.25)
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    plan = B.RK4Plan(B.Mesh(spec), B.default_params())
+    for t in (14, 15, 16):
+        assert plan.set_tile(t) == {13: 6}
+    _, table = plan.autotune(U, reps=1)
+    assert table[13][6] == table[13][4] and table[13][7] == table[13][3]
+    assert all(table[13][t] > 1e29 for t in (14, 15, 16))
+    plan.close()
