@@ -177,8 +177,7 @@ def _constraints(B, mesh, P, psi4, stream=None):
 def test_captured_constraints_outlive_scratch_growth(psi4):
     """Constraints captured on a mesh that already has derivative scratch,
     replayed after a plan and a right-hand side have replaced that scratch: the
-    graph holds nothing of the mesh that can be freed.  The mesh needs several
-    scratch-fuls of the pool's size on every side but 13.  The forms with and
+    graph holds nothing of the mesh that can be freed.  The forms with and
     without scratch round the outer stage of the mixed derivatives differently:
     1e-12 of the largest value."""
     import bssn_b200 as B
@@ -202,6 +201,27 @@ def test_captured_constraints_outlive_scratch_growth(psi4):
     torch.cuda.synchronize()
     assert ol.rel_err(eager.cpu().numpy(), captured.cpu().numpy()).max() <= 1e-12
     plan.close()
+
+
+def test_constraints_over_several_scratch_fuls():
+    """1.16 M zones of 13^3 blocks, more than one call's scratch holds, against
+    the form without scratch (as above)."""
+    import bssn_b200 as B
+    spec = B.generate_mesh(0, (15, 15, 15), seed=0, xmin=-8.25)
+    assert spec.zones() > 1 << 20
+    U = torch.zeros((24, spec.n_nodes), dtype=torch.float64, device="cuda")
+    B.initial_data(U, spec, eps=1e-6)
+    mesh = B.Mesh(spec)
+    P = torch.zeros((24, mesh.n_unzip), dtype=torch.float64, device="cuda")
+    mesh.unzip(P, U)
+    eager = _constraints(B, mesh, P, True)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        captured = _constraints(B, mesh, P, True)
+    g.replay()
+    torch.cuda.synchronize()
+    assert ol.rel_err(eager.cpu().numpy(), captured.cpu().numpy()).max() <= 1e-12
 
 
 def test_constraints_beside_right_hand_sides():

@@ -54,6 +54,21 @@ def test_wavelet_scores_vs_oracle(B, state):
     assert np.array_equal(flags.cpu().numpy(), (rmax / 1e-6 > 1.0).astype(np.uint8))
 
 
+@pytest.mark.parametrize("nvars", [1, 2, 3, 5, 22, 23])
+def test_wavelet_scores_of_some_variables(B, state, nvars):
+    """Variable counts that leave a warp's group of four part empty: the same
+    bits as those variables' scores among all 24."""
+    spec, m, Pz = state
+    every, _, _ = B.wavelet_scores(m, Pz)
+    scores, ratio, flags = B.wavelet_scores(m, Pz, tol=1e-6, nvars=nvars)
+    torch.cuda.synchronize()
+    assert torch.equal(scores.view(torch.int64), every[:, :nvars].contiguous().view(torch.int64))
+    first = np.cumsum([0] + [((int(s) - 7) // 6) ** 3 for s in spec.sides])
+    rmax = np.array([scores[first[b]:first[b + 1]].max().item() for b in range(spec.nblocks)])
+    assert np.array_equal(ratio.cpu().numpy(), rmax / 1e-6)
+    assert np.array_equal(flags.cpu().numpy(), (rmax / 1e-6 > 1.0).astype(np.uint8))
+
+
 def test_block_features_vs_oracle(B, state):
     spec, m, Pz = state
     f = B.block_features(m, Pz).cpu().numpy()
