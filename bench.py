@@ -71,7 +71,7 @@ FLOP_PER_ZONE_STAGE = 6535.0  # 6,439 RHS + 96 RK axpy (per zone, per stage)
 
 SPLIT_SLOTS = 162  # scratch doubles per zone of the split right-hand side
 KIND_NAMES = {"fused": "bssn::rhs_kernel / bssn::onchip_kernel (one-kernel right-hand side)",
-              "deriv": "bssn::column_kernel (derivative pass)", "eq": "bssn::eq_kernel (equation pass)"}
+              "deriv": "bssn::column_kernel / bssn::cube_kernel (derivative pass)", "eq": "bssn::eq_kernel (equation pass)"}
 
 
 def tile_pins(arg):
@@ -109,9 +109,10 @@ def kernel_bytes(sides, chosen, modes):
 # captures on small workloads (dram__bytes_read.sum + dram__bytes_write.sum
 # over the launch's algorithmic bytes as kernel_bytes counts them).  Scales a
 # full pass's algorithmic bytes to DRAM traffic; kinds without a capture of the
-# present kernel report none.  (uniform 512: eq 249.3 + 17.9 MB against
-# 384 * 343 * 512 B -- the scratch round trip is the excess)
-TRAFFIC_RATIO = {"eq": 267.2e6 / (384 * 343 * 512)}
+# present kernel report none.  (477 mixed blocks, one stage from the node grid:
+# derivative launches 1,554 MB for 192 s^3 B a block, equation launches 1,725 MB
+# for 384 B a zone -- the scratch round trip is the excess)
+TRAFFIC_RATIO = {"deriv": 1554.1e6 / 507359808, "eq": 1725.0e6 / (384 * 1039941)}
 
 
 def rhs_bytes(sides):
@@ -301,9 +302,10 @@ def run_reference(args, wl):
            "vs_baseline": None, "dtype": "f64", "data": "synthetic",
            "config": {"workload": name, "sampled_from": wl, "description": desc,
                       "blocks": c.spec.nblocks, "zones": zones, "nodes": c.spec.n_nodes,
-                      "path": "reference CPU RK4 step: oracle ghost fill + the reference's compiled "
-                              "bssnrhs block loop (OpenMP over blocks) + zip + stage algebra + "
-                              "enforce_bssn_constraints"},
+                      "path": "CPU RK4 step: oracle ghost fill + "
+                              + ("the reference's compiled bssnrhs" if c.kind == "reference" else
+                                 "the oracle's restatement of bssnrhs (no compiled reference here)")
+                              + " block loop (OpenMP over blocks) + zip + stage algebra + constraint enforcement"},
            "cpu_baseline": dict(info, value=rate, unit="zone-updates/s", cpu_model=cpu_model()),
            "e2e": {"value": rate, "unit": "zone-updates/s", "h2d_bytes_per_step": 0,
                    "d2h_bytes_per_step": 0},

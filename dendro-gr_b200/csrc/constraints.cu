@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(128) constraints_scratch_kernel(ConstVars P, M
     constraints_point<PSI4>(P, out, bd, at, node, dv);
 }
 
-// One CTA per chunk of up to 1024 interior points of a block, 256 threads
+// One CTA per chunk of interior points of a block (mesh.cu), 256 threads
 // striding over it (the node function needs up to 255 registers).
 template <bool PSI4>
 __global__ void __launch_bounds__(256) constraints_kernel(ConstVars P, MutVars out,

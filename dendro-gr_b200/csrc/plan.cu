@@ -1,6 +1,9 @@
-// The whole RK4 step as one plan: per stage a ghost fill (unzip), the fused
-// right-hand side over every brick of every block (one launch per block-size
-// bucket with that bucket's autotuned tile), and the zip fused with the stage
+// The whole RK4 step as one plan.  Per stage on single-level meshes: the
+// right-hand side of every block straight from the zipped state, written zipped
+// (per block-size bucket, with that bucket's tile, a derivative and an equation
+// launch for each scratch-full of bricks), and a node-wise kernel with the stage
+// algebra.  On level meshes, with a fused tile, or block by block: a ghost fill
+// (unzip), the right-hand side on padded blocks, and the zip fused with the stage
 // algebra.  Optionally captured once as a CUDA graph and replayed, or run as
 // the plain path with one right-hand-side launch per block (the structure of
 // the reference's bssnRHS block loop, rhs.cpp:10-73) for comparison.

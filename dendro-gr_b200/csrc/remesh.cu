@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(256) element_features_kernel(ConstVars U,
     }
 }
 
-// Block flags from element decisions, one warp per block: an element the
+// Block flags from element decisions, WARPS warps per block: an element the
 // exact test ran on (need) takes its flags from its largest score over the
 // variables (ratio = max / tol: refine above 1, keep above keep_fac), the
 // others the networks' decisions; a block refines (keeps) when any of its

@@ -23,9 +23,11 @@
 // one-sided closures and meet the others at the same barriers; next to a
 // physical z face a pass after the march redoes three zones.
 //
-// What bounds it: FP64 and shared-memory issue, and the barrier per plane.  A
-// zone and variable cost about 100 FP64 warp instructions per 32 zones and 23
-// shared loads of a thread's own; the form that this replaces (a cube of brick
+// What bounds it: the barrier per plane and shared-memory and FP64 issue
+// (barrier 3-5 of 9-12 stall cycles per issue, LSU data pipe 34-47 % and FP64 17-22 %
+// on a step of 477 mixed blocks, DRAM 20 %).  32 zones of a variable cost 102
+// (55^3) to 119 (19^3) FP64 warp instructions and 35 to 45 shared loads; the
+// form that this replaces (a cube of brick
 // + halo per variable, one thread per zone, mixed derivatives through a
 // cooperative halo pass, closures by per-term constant tables) issued about
 // 430 instructions with 52 shared loads.  Derivative passes of one RK4 step:
@@ -76,11 +78,12 @@ struct ColShape {
     static constexpr int COLS = BX * BY;
     static constexpr int PL = TX * TY;   // staged points of a plane
     static constexpr int DXP = BX * TY;  // d/dx of a plane, with the halo rows
-        // Two CTAs of 256 threads per SM at 128 registers, or, for full-width
-    // strips of 55^3 blocks, whose halo rows weigh more than a second CTA
+    // Two CTAs of at most 256 threads per SM (31^3: 256 at 128 registers, 19^3:
+    // 192 at 160), or, for full-width strips of 55^3 blocks, whose halo rows weigh more than a second CTA
     // gives, one of 512: derivative passes of one RK4 step on 98 such blocks
     // (10.8 M zones) 21.5 ms with 49 x 10 columns, 24.1 with 49 x 13 in 640
-    // threads, 26.7 with two CTAs of 49 x 5.
+    // threads, 26.7 with two CTAs of 49 x 5.  ITER, the staged points whose
+    // pointers a thread keeps, has not been swept.
     static constexpr int MAXT = BX >= 49 ? 512 : 256;
     static constexpr int MINB = BX >= 49 ? 1 : 2;
     static constexpr int ITER = BX >= 9 ? 3 : 4;

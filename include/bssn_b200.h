@@ -115,7 +115,8 @@ int bssn_mesh_destroy(bssn_mesh mesh);
  * offsets) = one past the largest offset + s^3 */
 int64_t bssn_mesh_unzip_size(bssn_mesh mesh);
 
-/* All blocks of a mesh in one launch.  Replaces bssnRHS(unzipVarsRHS,
+/* All blocks of a mesh: a derivative and an equation launch per block side (and
+ * scratch-full of bricks) with split tiles, one launch with the others.  Replaces bssnRHS(unzipVarsRHS,
  * uZipVars, blkList, numBlocks, t, uZipConstVars) (rhs.cpp:10-73) and the
  * GPU comparator device::bssnrhs3 (cuda/include/bssn_kernels.cuh:1526-1538).
  * tile: -1 = each block side's default split tile; otherwise a tile id in
